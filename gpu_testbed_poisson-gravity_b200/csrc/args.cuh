@@ -32,6 +32,7 @@ inline SolveArgs<T> make_args(const gpg_params &p, int64_t npatch, const void *r
   volatile T o6 = omega;
   o6 = o6 / (T)6.0;
   a.omega_6 = o6;
+  a.neg_zero = T(-0.0);
   a.gra_const = p.p5_gradient ? (T)((double)dt / (12.0 * (double)dh)) : (T)((double)dt / (2.0 * (double)dh));
   a.dh = dh;
   a.poi_coeff = poi;

@@ -83,6 +83,7 @@ struct SolveArgs {
   int64_t npatch;
   T sor_const;      // Poi_Coeff*dh*dh        (CPU_PoissonSolver_SOR.cpp:51)
   T omega_6;        // Omega/6                (CPU_PoissonSolver_SOR.cpp:52)
+  T neg_zero;       // -0.0, unknown to the compiler: fma(a, b, neg_zero) is a * b rounded on its own
   T gra_const;      // dt/(2dh) or dt/(12dh)  (CPU_GravitySolver.cpp:23)
   T dh;
   T poi_coeff;

@@ -455,11 +455,11 @@ __global__ void __launch_bounds__(Shape<HALVES, STAGE>::kThreads, 1) lin_sor_ker
       // interpolation and residual only: no sweeps, nothing else stored
       SolveArgs<float> s = a.s;
       s.max_iter = 0;
-      sor_solve_patch_with<float, 1, false, 2, 2>(s, P_, 0, lane, tb, false, hook);
+      sor_solve_patch_with<float, 1, false, 2, 2, false, false>(s, P_, 0, lane, tb, false, hook);
     } else if constexpr (kStaged) {
-      sor_solve_patch_with<float, 1, false, 2, 2, true>(a.s, P_, 0, lane, tb, real, hook, stg);
+      sor_solve_patch_with<float, 1, false, 2, 2, true, false>(a.s, P_, 0, lane, tb, real, hook, stg);
     } else {
-      sor_solve_patch_with<float, 1, false, 2, 2>(a.s, P_, 0, lane, tb, real, hook);
+      sor_solve_patch_with<float, 1, false, 2, 2, false, false>(a.s, P_, 0, lane, tb, real, hook);
     }
   }
   if constexpr (!FEATURES) {

@@ -303,6 +303,198 @@ __device__ __forceinline__ void sor_pass2(T (&v)[2][2][SorCfg<T, G, Z, 2>::MH + 
   }
 }
 
+// ---------------------------------------------------------------------------
+// FP32, two rows per lane: the same pass with two heights of a row in one
+// packed register pair (add / fma .f32x2: one instruction, two IEEE roundings).
+// The scalar kernels filled 74 % of the issue slots (ghost 3, 4096 patches), and
+// ten of an update's thirteen instructions are these ordered operations.  20
+// sweeps with residual sums: 172 -> 156 us at ghost 3; without sums the sweeps
+// run at the shared-memory pipe's pace either way (4.3 us each).  Whole solves of
+// 4096 patches, scalar -> packed: ghost 2 65.9 -> 58.9 us, 3 115.2 -> 106.9, 4
+// 168.0 -> 152.6, 5 231.3 -> 202.5; the mixed-size work-queue kernel 2.37 -> 1.82
+// ms for 65,536 patches.
+//
+// A multiplication is fma(a, b, -0) with the -0 read from the kernel
+// arguments: exactly the rounded product (also in the sign of a zero), and
+// nothing that an optimiser could merge with the addition after it.
+//
+// Pairs: heights z and z+2 (groups of four: (1,3), (2,4), ...), so that both
+// cells of a pair sit on the same side of their x-pair and the x operands need
+// no shuffling; the in-lane y neighbours and the x mates are pairs of the
+// other colour at the same two heights.  Only the first addition, z+1 with
+// z-1, mixes pairs and stays scalar.  Heights left over: two make a pair of
+// opposite sides (scalar x additions), one stays scalar.
+// ---------------------------------------------------------------------------
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float lo2(f32x2 v) {
+  float a, b;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+  return a;
+}
+__device__ __forceinline__ float hi2(f32x2 v) {
+  float a, b;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+  return b;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+template <int MH>
+struct PackPairs {
+  static constexpr int QUADS = MH / 4, REM = MH % 4;
+  static constexpr int NP = 2 * QUADS + (REM >= 2 ? 1 : 0);  // pairs per row and colour
+  static constexpr int NS = REM & 1;                         // single heights
+  static constexpr int SINGLE = REM == 3 ? 4 * QUADS + 2 : 4 * QUADS + 1;
+  __host__ __device__ static constexpr int lo(int k) { return 4 * (k / 2) + 1 + (k & 1); }
+  __host__ __device__ static constexpr int hi(int k) { return lo(k) + (same_side(k) ? 2 : 1); }
+  __host__ __device__ static constexpr bool same_side(int k) { return k < 2 * QUADS || REM == 3; }
+  // pair of height z (1..MH, not the single one), and whether z is its low half
+  __host__ __device__ static constexpr int pair_of(int z) {
+    return z > 4 * QUADS ? 2 * QUADS : 2 * ((z - 1) / 4) + ((z - 1) & 1);
+  }
+  __host__ __device__ static constexpr bool is_lo(int z) { return lo(pair_of(z)) == z; }
+};
+
+// A lane's columns in packed form, [row][colour]: value pairs, the height
+// that stays single, the values below and above the column, -Const*rho.
+template <int MH>
+struct PackState {
+  using PK = PackPairs<MH>;
+  f32x2 v[2][2][PK::NP], nc[2][2][PK::NP];
+  float s[2][2], ncs[2][2];
+  float below[2][2], above[2][2];
+  __device__ __forceinline__ float at(int r, int c, int z) const {
+    if (z == 0) return below[r][c];
+    if (z == MH + 1) return above[r][c];
+    if (PK::NS && z == PK::SINGLE) return s[r][c];
+    const f32x2 q = v[r][c][PK::pair_of(z)];
+    return PK::is_lo(z) ? lo2(q) : hi2(q);
+  }
+  template <typename V, typename R>
+  __device__ __forceinline__ void load(const V &x, const R &crho) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+#pragma unroll
+        for (int k = 0; k < PK::NP; ++k) {
+          v[r][c][k] = pack2(x[r][c][PK::lo(k)], x[r][c][PK::hi(k)]);
+          nc[r][c][k] = pack2(-crho[r][c][PK::lo(k) - 1], -crho[r][c][PK::hi(k) - 1]);
+        }
+        if constexpr (PK::NS) {
+          s[r][c] = x[r][c][PK::SINGLE];
+          ncs[r][c] = -crho[r][c][PK::SINGLE - 1];
+        }
+        below[r][c] = x[r][c][0];
+        above[r][c] = x[r][c][MH + 1];
+      }
+  }
+};
+
+template <int G, int Z, bool PHASED, int p, bool SUM, int SIDE>
+__device__ __forceinline__ void sor_pass2_packed(PackState<SorCfg<float, G, Z, 2>::MH> &st, float *s_cube,
+                                                 const SorLane &ln, float omega_6, float neg_zero,
+                                                 double (&acc4)[4]) {
+  using C = SorCfg<float, G, Z, 2>;
+  constexpr int N = Geo<G>::N, MH = C::MH, P = C::P, PP = C::PP;
+  using PK = PackPairs<MH>;
+  constexpr int q = 1 - p;
+  const float *nb = s_cube + q * N * PP + ln.zoff;
+  float *mine = s_cube + p * N * PP + ln.zoff;
+  const f32x2 nz = pack2(neg_zero, neg_zero), w2 = pack2(omega_6, omega_6), m6 = pack2(-6.f, -6.f);
+  if constexpr (Z == 2) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const float b = nb[(ln.zh ? 0 : MH + 1) * PP + ln.own + r * P];
+      if (ln.zh)
+        st.below[r][q] = b;
+      else
+        st.above[r][q] = b;
+    }
+  }
+  constexpr bool RT = (Z == 2) && (MH & 1);
+  const bool le = SIDE >= 0 ? SIDE == 1 : (RT ? ln.left_even : true);
+  auto left_of = [&](int r, int z) { return ((((z + p) & 1) == 0) == le) == (r == 1); };
+  auto z_sum = [&](int r, int z) { return add(st.at(r, q, z + 1), st.at(r, q, z - 1)); };
+  auto y_smem = [&](int r, int z) { return nb[z * PP + ln.own + (r ? 2 * P : -P)]; };
+  auto x_out = [&](int r, int z) { return nb[z * PP + ln.own + r * P + (left_of(r, z) ? -1 : 1)]; };
+  auto store = [&](int r, int z, float x) { mine[z * PP + ln.own + r * P] = x; };
+  auto total = [&](int r, int z, float x) {
+    if constexpr (SUM) acc4[(z + 2 * r) & 3] += (double)absval(x);
+  };
+  // the six neighbours of the pair's two cells, in the reference's order
+  auto pair_sum = [&](int r, int k) -> f32x2 {
+    const int a = PK::lo(k), b = PK::hi(k);
+    f32x2 t = pack2(z_sum(r, a), z_sum(r, b));
+    const f32x2 yreg = st.v[1 - r][q][k], ysm = pack2(y_smem(r, a), y_smem(r, b));
+    t = add2(add2(t, r == 0 ? yreg : ysm), r == 0 ? ysm : yreg);
+    const f32x2 mate = st.v[r][q][k];
+    const float xa = x_out(r, a), xb = x_out(r, b);
+    if (PK::same_side(k)) {
+      const f32x2 xo = pack2(xa, xb);
+      const bool left = left_of(r, a);
+      return add2(add2(t, left ? mate : xo), left ? xo : mate);
+    }
+    const bool la = left_of(r, a), lb = left_of(r, b);
+    const float ta = add(add(lo2(t), la ? lo2(mate) : xa), la ? xa : lo2(mate));
+    const float tb = add(add(hi2(t), lb ? hi2(mate) : xb), lb ? xb : hi2(mate));
+    return pack2(ta, tb);
+  };
+  auto pair_update = [&](int r, int k, f32x2 sum) {
+    const f32x2 res = add2(add2(sum, fma2(m6, st.v[r][p][k], nz)), st.nc[r][p][k]);
+    st.v[r][p][k] = add2(st.v[r][p][k], fma2(w2, res, nz));
+    total(r, PK::lo(k), lo2(res));
+    total(r, PK::hi(k), hi2(res));
+  };
+  if constexpr (PHASED) {
+    f32x2 sum[2][PK::NP];
+#pragma unroll
+    for (int k = 0; k < PK::NP; ++k)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) sum[r][k] = pair_sum(r, k);
+#pragma unroll
+    for (int k = 0; k < PK::NP; ++k)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) pair_update(r, k, sum[r][k]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < PK::NP; ++k)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) pair_update(r, k, pair_sum(r, k));
+  }
+  if constexpr (PK::NS) {
+    constexpr int z = PK::SINGLE;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const float yreg = st.s[1 - r][q], ysm = y_smem(r, z), xo = x_out(r, z), mate = st.s[r][q];
+      const bool left = left_of(r, z);
+      float t = add(add(z_sum(r, z), r == 0 ? yreg : ysm), r == 0 ? ysm : yreg);
+      t = add(add(t, left ? mate : xo), left ? xo : mate);
+      const float res = add(sub(t, mul(6.f, st.s[r][p])), st.ncs[r][p]);
+      st.s[r][p] = add(st.s[r][p], mul(omega_6, res));
+      total(r, z, res);
+    }
+  }
+#pragma unroll
+  for (int z = 1; z <= MH; ++z) {
+    store(0, z, st.at(0, p, z));
+    store(1, z, st.at(1, p, z));
+  }
+}
+
 template <typename T, int G, int Z, int Y, bool PHASED, int p, bool SUM>
 __device__ __forceinline__ void sor_pass_any(T (&v)[Y][2][SorCfg<T, G, Z, Y>::MH + 2],
                                              const T (&crho)[Y][2][SorCfg<T, G, Z, Y>::MH], T *s_cube,
@@ -348,8 +540,10 @@ struct SorLaneState {
 // team synchronised.  store == false skips every global write (a team that
 // only keeps a CTA-wide schedule going).  STAGED: the patch's coarse
 // potential and density come from `staged` in shared memory ([POT_NXT]^3
-// then [RHO_NXT]^3) instead of global memory.
-template <typename T, int G, bool PHASED, int Z, int Y, bool STAGED = false, typename Hook>
+// then [RHO_NXT]^3) instead of global memory.  PACK: FP32 two-row layouts
+// sweep in packed pairs (off where a solve takes about one sweep, which does not
+// pay for building them).
+template <typename T, int G, bool PHASED, int Z, int Y, bool STAGED = false, bool PACK = true, typename Hook>
 __device__ __forceinline__ void sor_solve_patch_with(const SolveArgs<T> &a, int64_t P_, int team, int tid,
                                                      unsigned char *tb, bool store, Hook &&hook,
                                                      const T *staged = nullptr) {
@@ -452,6 +646,9 @@ __device__ __forceinline__ void sor_solve_patch_with(const SolveArgs<T> &a, int6
 
   // ---- SOR sweeps ---------------------------------------------------------
   const T omega_6 = a.omega_6;
+  constexpr bool PACKED = PACK && Y == 2 && sizeof(T) == 4;
+  PackState<MH> packed;
+  if constexpr (PACKED) packed.load(v, crho);
   double total_old = (double)FLT_MAX, last = 0.0;
   int iter;
   for (iter = 0; iter < a.max_iter; ++iter) {
@@ -463,16 +660,35 @@ __device__ __forceinline__ void sor_solve_patch_with(const SolveArgs<T> &a, int6
     // combined in a fixed order, so the total is deterministic and identical
     // for a patch solved alone or in a batch
     double acc4[4] = {0.0, 0.0, 0.0, 0.0};
+    auto pass = [&](auto colour_c, auto sum_c) {
+      constexpr int p = decltype(colour_c)::value;
+      constexpr bool SUM = decltype(sum_c)::value;
+      if (!active) return;
+      if constexpr (PACKED) {
+        if constexpr (C::HALF_UNIFORM) {
+          if (ln.left_even)  // warp-uniform branch
+            sor_pass2_packed<G, Z, PHASED, p, SUM, 1>(packed, s_cube, ln, omega_6, a.neg_zero, acc4);
+          else
+            sor_pass2_packed<G, Z, PHASED, p, SUM, 0>(packed, s_cube, ln, omega_6, a.neg_zero, acc4);
+        } else {
+          sor_pass2_packed<G, Z, PHASED, p, SUM, -1>(packed, s_cube, ln, omega_6, a.neg_zero, acc4);
+        }
+      } else {
+        sor_pass_any<T, G, Z, Y, PHASED, p, SUM>(v, crho, s_cube, ln, omega_6, acc4);
+      }
+    };
+    constexpr std::integral_constant<int, 0> first{};
+    constexpr std::integral_constant<int, 1> second{};
     if (!need) {
-      if (active) sor_pass_any<T, G, Z, Y, PHASED, 0, false>(v, crho, s_cube, ln, omega_6, acc4);
+      pass(first, std::false_type{});
       team_sync<TEAM>(team);
-      if (active) sor_pass_any<T, G, Z, Y, PHASED, 1, false>(v, crho, s_cube, ln, omega_6, acc4);
+      pass(second, std::false_type{});
       team_sync<TEAM>(team);
       continue;
     }
-    if (active) sor_pass_any<T, G, Z, Y, PHASED, 0, true>(v, crho, s_cube, ln, omega_6, acc4);
+    pass(first, std::true_type{});
     team_sync<TEAM>(team);
-    if (active) sor_pass_any<T, G, Z, Y, PHASED, 1, true>(v, crho, s_cube, ln, omega_6, acc4);
+    pass(second, std::true_type{});
     double acc = (acc4[0] + acc4[1]) + (acc4[2] + acc4[3]);
     acc = warp_sum(acc);
     if constexpr (NWARP > 1) {

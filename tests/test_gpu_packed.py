@@ -1,0 +1,50 @@
+"""FP32 two-row SOR kernels sweep two heights per packed register pair: their
+results must be those of the scalar one-row kernel (variant 0) bit for bit,
+also where values are zeros of either sign, denormal or not finite, and at
+patch counts around a launch's tail (needs a B200)."""
+import numpy as np
+import pytest
+
+from gpg.abi import GPG_SOR, default_params
+from gpg.inputs import make_patches
+
+pytestmark = pytest.mark.gpu
+
+
+def special_patches(npatch, g):
+    d = make_patches(npatch, g, seed=40 + g, dtype=np.float32, fluid=False)
+    rho, pin = d["rho"], d["pot_in"]
+    rho[0], pin[0] = 0.0, 0.0
+    if npatch > 1:
+        rho[1], pin[1] = -0.0, -0.0
+    if npatch > 2:
+        rho[2] *= np.float32(1e-38)
+        pin[2] *= np.float32(1e-40)
+    if npatch > 3:
+        rho[3, 1, 2, 3] = np.nan
+    if npatch > 4:
+        pin[4, 3, 3, 3] = np.inf
+    return rho, pin
+
+
+@pytest.mark.parametrize("g", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("npatch", [1, 149, 331])
+def test_packed_kernels_return_the_scalar_bits(g, npatch):
+    torch = pytest.importorskip("torch")
+    from gpg.lib import check, library, solve_device
+    lib, dev = library(), torch.device("cuda:0")
+    rho, pin = (torch.from_numpy(a).to(dev) for a in special_patches(npatch, g))
+    p = default_params(4, g, GPG_SOR, gra_acc=0, sor_max_iter=23)
+    outs = {}
+    try:
+        for v in (0, 10, 11, 12, 13, 14, 15, 16):
+            check(lib.gpg_set_sor_variant(4, g, v))
+            pot, _, it, rs = solve_device(p, rho, pin)
+            outs[v] = [pot.view(torch.int32).cpu(), torch.isnan(pot).cpu(), it.cpu(), rs.cpu()]
+    finally:
+        check(lib.gpg_set_sor_variant(4, g, -1))
+    bits0, nan0, it0, rs0 = outs[0]
+    for v, (bits, nan, it, rs) in outs.items():
+        assert torch.equal(nan, nan0) and torch.equal(it, it0), v
+        assert torch.equal(bits[~nan], bits0[~nan0]), v  # a NaN's payload is not specified
+        assert torch.equal(torch.nan_to_num(rs, nan=-1.0), torch.nan_to_num(rs0, nan=-1.0)), v
