@@ -647,7 +647,8 @@ int adam_step(gpg_net *n, const float *grad, float lr, cudaStream_t s) {
   n->step += 1;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - std::pow(b1, float(n->step)), c2 = 1.f - std::pow(b2, float(n->step));
-  gpg::adam_kernel<<<128, 256, 0, s>>>(n->params, n->adam_m, n->adam_v, grad, kParams, lr, b1, b2, 1e-8f, c1, c2);
+  gpg::adam_kernel<<<128, 256, 0, s>>>(
+      gpg::AdamArgs{n->params, n->adam_m, n->adam_v, grad, lr, b1, b2, 1e-8f, c1, c2}, kParams);
   NET_CUDA(cudaGetLastError());
   return repack(n, s);
 }

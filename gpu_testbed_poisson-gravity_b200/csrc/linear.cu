@@ -15,6 +15,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -55,69 +56,185 @@ int lfail(int status, const char *fmt, ...) {
 // class of block b: number of odd axes
 __host__ __device__ constexpr int class_of(int b) { return (b & 1) + ((b >> 1) & 1) + ((b >> 2) & 1); }
 
-// W[4][64][64] (FP32) -> the two stacked A tiles [kc][row 0..127][8] (BF16):
-// tile 0 = (class 0 ; class 3), tile 1 = (class 1 ; class 2)
+// four consecutive values, in one 128-bit load where the pointer allows it
+__device__ __forceinline__ float4 load4(const float *p) {
+  if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) return __ldg(reinterpret_cast<const float4 *>(p));
+  return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+}
+
+// place of parameter i = (class, row, k) in the two stacked A tiles
+// [kc][row 0..127][8]: tile 0 = (class 0 ; class 3), tile 1 = (class 1 ; class 2)
+__device__ __forceinline__ int tile_index(int i) {
+  const int cls = i / (kK * kK), r = (i / kK) % kK, k = i % kK;
+  const int t = (cls == 1 || cls == 2) ? 1 : 0, row = r + (cls >= 2 ? kK : 0);
+  return t * 128 * kK + ((k >> 3) * 128 + row) * 8 + (k & 7);
+}
+
+// W[4][64][64] (FP32) -> the A tiles (BF16)
 __global__ void lin_pack_kernel(const float *__restrict__ w, __nv_bfloat16 *__restrict__ tiles) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 2 * 128 * kK; i += gridDim.x * blockDim.x) {
-    const int t = i / (128 * kK), rem = i - t * 128 * kK;
-    const int kc = rem / (128 * 8), row = (rem / 8) % 128, e = rem % 8;
-    const int cls = t == 0 ? (row < 64 ? 0 : 3) : (row < 64 ? 1 : 2);
-    tiles[i] = __float2bfloat16_rn(w[(cls * kK + (row & 63)) * kK + kc * 8 + e]);
-  }
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < kParams) tiles[tile_index(i)] = __float2bfloat16_rn(w[i]);
 }
 
-// per patch (one CTA of 512 threads = 8 blocks x 64 rows): the errors
-// e = W u - t and the patch's sum of e^2 (fixed-order tree)
-__global__ void __launch_bounds__(512) lin_err_kernel(const float *__restrict__ u, const float *__restrict__ t,
-                                                      const float *__restrict__ w, float *__restrict__ e,
-                                                      float *__restrict__ loss_part) {
-  __shared__ float su[512];
-  __shared__ float red[512];
-  const int p = blockIdx.x, tid = threadIdx.x, b = tid >> 6, r = tid & 63;
-  su[tid] = u[int64_t(p) * 512 + tid];
-  __syncthreads();
-  const float *wr = w + (class_of(b) * kK + r) * kK;
-  const float *ub = su + b * kK;
-  float acc = 0.f;
-#pragma unroll 8
-  for (int k = 0; k < kK; ++k) acc = fmaf(__ldg(wr + k), ub[k], acc);
-  const float err = acc - t[int64_t(p) * 512 + tid];
-  e[int64_t(p) * 512 + tid] = err;
-  red[tid] = err * err;
-  __syncthreads();
-  for (int h = 256; h > 0; h >>= 1) {
-    if (tid < h) red[tid] += red[tid + h];
-    __syncthreads();
-  }
-  if (tid == 0) loss_part[p] = red[0];
+// one Adam step and the operand tiles of the new weights
+__global__ void lin_adam_kernel(const gpg::AdamArgs a, __nv_bfloat16 *__restrict__ tiles) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < kParams) tiles[tile_index(i)] = __float2bfloat16_rn(gpg::adam_update(a, i));
 }
 
-// grad[c][r][k] = 2 / (npatch 512) sum_p sum_{b in c} e[p][b][r] u[p][b][k]
-// (CTA = class c, 4 rows; thread = (row, k); patches and blocks in order)
-__global__ void __launch_bounds__(256) lin_grad_kernel(const float *__restrict__ us, const float *__restrict__ e,
-                                                       int npatch, float *__restrict__ grad) {
-  const int c = blockIdx.x / 16, r = (blockIdx.x % 16) * 4 + (threadIdx.x >> 6), k = threadIdx.x & 63;
-  float acc = 0.f;
-  for (int p = 0; p < npatch; ++p)
+// ---------------------------------------------------------------------------
+// Gradient of the loss.  Two dense FP32 products per block b of class c,
+//   E = W[c] U^T - T    (64 rows x patches),    G = E U    (64 x 64),
+// 0.27 GFLOP for 2048 patches (3.6 us at the FP32 peak) over 8.4 MB of
+// features.  CTA (b, j) takes the patches j, j + grid.y, ... in chunks of 64:
+// W[c] transposed stays in shared memory, E lives there between the two
+// products (each thread 4 rows x 4 patches, then 4 rows x 4 columns), and the
+// CTA's G stays in registers until its chunks are done; the next chunk's
+// features are loaded while the current one is multiplied.  grid.y = 37 puts
+// two CTAs on each of 148 SMs (8 x 37 = 296) and bounds the partial sums to 4.8
+// MB, which the second kernel adds in a fixed order.
+// Training step (gradient, Adam, operand tiles) of 2048 patches: 1212 -> 24.6
+// us, of which the host's calls are about 22 (64 patches take the same).
+// (A thread that walks all patches for its row and column, as before, waits
+// for 6144 dependent steps.)
+// The error e = W u - t sums k in order, as the single-row form did.
+// ---------------------------------------------------------------------------
+constexpr int kGradSplit = 37;               // CTAs that share a block's patches
+constexpr int kChunk = 64;                   // patches per step
+constexpr int kGradThreads = 256;
+constexpr int kPitchW = kK + 4;              // row pitches (words) that keep the 128-bit accesses aligned
+struct GradSmem {
+  float wt[kK][kPitchW];                     // W[c]^T: [k][row]
+  float u[kChunk][kPitchW];                  // [patch][k]
+  float e[kChunk][kPitchW];                  // [patch][row]
+  double loss[kGradThreads / 32];
+};
+
+__global__ void __launch_bounds__(kGradThreads) lin_grad_kernel(const float *__restrict__ u,
+                                                                const float *__restrict__ t,
+                                                                const float *__restrict__ w, int npatch,
+                                                                float *__restrict__ part,
+                                                                double *__restrict__ loss_part) {
+  extern __shared__ __align__(16) unsigned char lin_smem[];
+  GradSmem &sm = *reinterpret_cast<GradSmem *>(lin_smem);
+  const int b = blockIdx.x, tid = threadIdx.x, c = class_of(b);
+  for (int i = tid; i < kK * kK; i += kGradThreads) sm.wt[i % kK][i / kK] = w[c * kK * kK + i];
+  const int r0 = (tid & 15) * 4;             // 4 rows of E and of G
+  const int p0 = (tid >> 4) * 4;             // 4 patches of E
+  const int k0 = p0;                         // 4 columns of G
+  float g[4][4] = {};
+  double loss = 0.0;
+  constexpr int NQ = kChunk * kK / 4 / kGradThreads;
+  const int64_t step = int64_t(gridDim.y) * kChunk;
+  float4 next[NQ];
+  auto fetch = [&](int64_t from) {  // this thread's share of the chunk at `from`
 #pragma unroll
-    for (int b = 0; b < 8; ++b)
-      if (class_of(b) == c) acc = fmaf(e[(int64_t(p) * 8 + b) * kK + r], us[(int64_t(p) * 8 + b) * kK + k], acc);
-  grad[(c * kK + r) * kK + k] = acc * (2.f / (float(npatch) * 512.f));
+    for (int q = 0; q < NQ; ++q) {
+      const int i = tid + q * kGradThreads, p = i / (kK / 4), k = (i % (kK / 4)) * 4;
+      next[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (from + p < npatch) next[q] = load4(u + ((from + p) * 8 + b) * kK + k);
+    }
+  };
+  fetch(int64_t(blockIdx.y) * kChunk);
+  for (int64_t first = int64_t(blockIdx.y) * kChunk; first < npatch; first += step) {
+    __syncthreads();  // the previous chunk's u and e are read; wt is written
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      const int i = tid + q * kGradThreads;
+      *reinterpret_cast<float4 *>(&sm.u[i / (kK / 4)][(i % (kK / 4)) * 4]) = next[q];
+    }
+    float4 want[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      want[q] = first + p0 + q < npatch ? load4(t + ((first + p0 + q) * 8 + b) * kK + r0)
+                                        : make_float4(0.f, 0.f, 0.f, 0.f);
+    fetch(first + step);
+    __syncthreads();
+    float e[4][4] = {};
+#pragma unroll 4
+    for (int k = 0; k < kK; k += 4) {
+      float x[4][4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<float4 *>(x[q]) = *reinterpret_cast<const float4 *>(&sm.u[p0 + q][k]);
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        const float4 wk = *reinterpret_cast<const float4 *>(&sm.wt[k + kk][r0]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          e[q][0] = fmaf(wk.x, x[q][kk], e[q][0]);
+          e[q][1] = fmaf(wk.y, x[q][kk], e[q][1]);
+          e[q][2] = fmaf(wk.z, x[q][kk], e[q][2]);
+          e[q][3] = fmaf(wk.w, x[q][kk], e[q][3]);
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (first + p0 + q < npatch) {
+        const float4 x = want[q];
+        d = make_float4(e[q][0] - x.x, e[q][1] - x.y, e[q][2] - x.z, e[q][3] - x.w);
+        loss += double(d.x) * d.x + double(d.y) * d.y + (double(d.z) * d.z + double(d.w) * d.w);
+      }
+      *reinterpret_cast<float4 *>(&sm.e[p0 + q][r0]) = d;
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (int p = 0; p < kChunk; ++p) {
+      const float4 x = *reinterpret_cast<const float4 *>(&sm.e[p][r0]);
+      const float4 y = *reinterpret_cast<const float4 *>(&sm.u[p][k0]);
+      const float xe[4] = {x.x, x.y, x.z, x.w}, yu[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) g[i][j] = fmaf(xe[i], yu[j], g[i][j]);
+    }
+  }
+  const int slot = blockIdx.y * 8 + b;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    *reinterpret_cast<float4 *>(part + (int64_t(slot) * kK + r0 + i) * kK + k0) =
+        make_float4(g[i][0], g[i][1], g[i][2], g[i][3]);
+  loss = gpg::warp_sum(loss);
+  if ((tid & 31) == 0) sm.loss[tid >> 5] = loss;
+  __syncthreads();
+  if (tid == 0) {
+    double s = 0.0;
+    for (int q = 0; q < kGradThreads / 32; ++q) s += sm.loss[q];
+    loss_part[slot] = s;
+  }
 }
 
-// loss = sum_p loss_part[p] / (npatch 512), fixed order (one CTA)
-__global__ void __launch_bounds__(256) lin_loss_kernel(const float *__restrict__ part, int npatch,
-                                                       float *__restrict__ loss) {
-  __shared__ double red[256];
-  double s = 0.0;
-  for (int p = threadIdx.x; p < npatch; p += 256) s += part[p];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int h = 128; h > 0; h >>= 1) {
-    if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
-    __syncthreads();
+// grad[c] = 2 / (npatch 512) sum of its blocks' partial sums; the loss from
+// the same kernel's partials (fixed orders).  Four threads share a value's
+// partials, so that no thread waits for more than ten loads of a block.
+__global__ void __launch_bounds__(256) lin_reduce_kernel(const float *__restrict__ part,
+                                                         const double *__restrict__ loss_part, int nsplit, int npatch,
+                                                         float *__restrict__ grad, float *__restrict__ loss) {
+  __shared__ float sums[4][64];
+  const int v = threadIdx.x & 63, q = threadIdx.x >> 6, i = blockIdx.x * 64 + v;
+  const int c = i / (kK * kK), rk = i % (kK * kK);
+  float s = 0.f;
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    if (class_of(b) != c) continue;
+    float x[(kGradSplit + 3) / 4];  // all loads of a block in flight together
+#pragma unroll
+    for (int j = 0; j < (kGradSplit + 3) / 4; ++j)
+      x[j] = q + 4 * j < nsplit ? part[int64_t((q + 4 * j) * 8 + b) * kK * kK + rk] : 0.f;
+#pragma unroll
+    for (int j = 0; j < (kGradSplit + 3) / 4; ++j) s += x[j];
   }
-  if (threadIdx.x == 0) *loss = float(red[0] / (double(npatch) * 512.0));
+  sums[q][v] = s;
+  __syncthreads();
+  if (q == 0) grad[i] = ((sums[0][v] + sums[1][v]) + (sums[2][v] + sums[3][v])) * (2.f / (float(npatch) * 512.f));
+  if (blockIdx.x == 0 && threadIdx.x < 32) {
+    double l = 0.0;
+    for (int j = threadIdx.x; j < nsplit * 8; j += 32) l += loss_part[j];
+    l = gpg::warp_sum(l);
+    if (threadIdx.x == 0) *loss = float(l / (double(npatch) * 512.0));
+  }
 }
 
 }  // namespace
@@ -128,7 +245,8 @@ struct gpg_lin {
   int step = 0;
   int probe_polls = 0;
   float *params = nullptr, *grad = nullptr, *adam_m = nullptr, *adam_v = nullptr;
-  float *e = nullptr, *loss_part = nullptr, *loss = nullptr;
+  float *part = nullptr, *loss = nullptr;  // partial gradients [kGradSplit * 8][64][64]
+  double *loss_part = nullptr;
   __nv_bfloat16 *tiles = nullptr;
   int *err = nullptr;
   int variant = 0;                   // launch shape of the fused solve
@@ -138,7 +256,7 @@ struct gpg_lin {
 namespace {
 
 int repack(gpg_lin *l, cudaStream_t s) {
-  lin_pack_kernel<<<32, 256, 0, s>>>(l->params, l->tiles);
+  lin_pack_kernel<<<kParams / 256, 256, 0, s>>>(l->params, l->tiles);
   LIN_CUDA(cudaGetLastError());
   return GPG_OK;
 }
@@ -213,8 +331,8 @@ extern "C" int gpg_lin_create(gpg_lin **out, int max_batch, int device_id) {
   al((void **)&l->adam_m, kParams * 4);
   al((void **)&l->adam_v, kParams * 4);
   al((void **)&l->tiles, 2 * gpg::lin::kTileBytes);
-  al((void **)&l->e, size_t(max_batch) * 512 * 4);
-  al((void **)&l->loss_part, size_t(max_batch) * 4);
+  al((void **)&l->part, size_t(kGradSplit) * 8 * kK * kK * 4);
+  al((void **)&l->loss_part, size_t(kGradSplit) * 8 * 8);
   al((void **)&l->loss, 4);
   al((void **)&l->err, 4);
   if (e == cudaSuccess) e = cudaMemset(l->params, 0, kParams * 4);
@@ -229,6 +347,9 @@ extern "C" int gpg_lin_create(gpg_lin **out, int max_batch, int device_id) {
   int rc = prepare<false, 2, true>(&l->grid[0]);
   if (!rc) rc = prepare<false, 3, false>(&l->grid[1]);
   if (!rc) rc = prepare<true, 2, false>(nullptr);
+  if (!rc && cudaFuncSetAttribute(lin_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  int(sizeof(GradSmem))) != cudaSuccess)
+    rc = lfail(GPG_ERR_CUDA, "shared memory of the gradient kernel: %s", cudaGetErrorString(cudaGetLastError()));
   if (rc) {
     gpg_lin_destroy(l);
     return rc;
@@ -246,7 +367,7 @@ extern "C" int gpg_lin_destroy(gpg_lin *l) {
   if (!l) return GPG_OK;
   cudaSetDevice(l->device);
   for (void *p : {(void *)l->params, (void *)l->grad, (void *)l->adam_m, (void *)l->adam_v, (void *)l->tiles,
-                  (void *)l->e, (void *)l->loss_part, (void *)l->loss, (void *)l->err})
+                  (void *)l->part, (void *)l->loss_part, (void *)l->loss, (void *)l->err})
     cudaFree(p);
   delete l;
   return GPG_OK;
@@ -336,9 +457,10 @@ extern "C" int gpg_lin_gradients(gpg_lin *l, int npatch, const float *d_u, const
   if (!d_u || !d_t) return lfail(GPG_ERR_INVALID, "NULL array");
   LIN_CUDA(cudaSetDevice(l->device));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  lin_err_kernel<<<npatch, 512, 0, s>>>(d_u, d_t, l->params, l->e, l->loss_part);
-  lin_grad_kernel<<<64, 256, 0, s>>>(d_u, l->e, npatch, d_grad ? d_grad : l->grad);
-  lin_loss_kernel<<<1, 256, 0, s>>>(l->loss_part, npatch, d_loss ? d_loss : l->loss);
+  const int nsplit = std::min(kGradSplit, (npatch + kChunk - 1) / kChunk);
+  lin_grad_kernel<<<dim3(8, nsplit), kGradThreads, sizeof(GradSmem), s>>>(d_u, d_t, l->params, npatch, l->part, l->loss_part);
+  lin_reduce_kernel<<<kParams / 64, 256, 0, s>>>(l->part, l->loss_part, nsplit, npatch, d_grad ? d_grad : l->grad,
+                                                  d_loss ? d_loss : l->loss);
   LIN_CUDA(cudaGetLastError());
   return GPG_OK;
 }
@@ -348,9 +470,10 @@ int lin_adam(gpg_lin *l, const float *grad, float lr, cudaStream_t s) {
   l->step += 1;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - std::pow(b1, float(l->step)), c2 = 1.f - std::pow(b2, float(l->step));
-  gpg::adam_kernel<<<64, 256, 0, s>>>(l->params, l->adam_m, l->adam_v, grad, kParams, lr, b1, b2, 1e-8f, c1, c2);
+  lin_adam_kernel<<<kParams / 256, 256, 0, s>>>(
+      gpg::AdamArgs{l->params, l->adam_m, l->adam_v, grad, lr, b1, b2, 1e-8f, c1, c2}, l->tiles);
   LIN_CUDA(cudaGetLastError());
-  return repack(l, s);
+  return GPG_OK;
 }
 }  // namespace
 
