@@ -26,6 +26,8 @@
 using gpg::net::ConvArgs;
 using gpg::net::WgradArgs;
 using gpg::net::kCells;
+using gpg::net::kEdge;
+using gpg::net::plane_elems;
 
 namespace {
 
@@ -69,28 +71,23 @@ constexpr int64_t kParams = param_offset_w(kLayers);
 // small kernels
 // ---------------------------------------------------------------------------
 
-// interpolated 10^3 cube of a ghost-1 patch (the SOR's initial cube)
-__global__ void __launch_bounds__(128) interp_cube_kernel(const float *__restrict__ pot_in, float *__restrict__ cube,
-                                                          int64_t npatch) {
-  const int64_t p = blockIdx.x;
-  if (p >= npatch) return;
-  float *dst = cube + p * kCells;
-  gpg::interpolate<float, 1, 128>(pot_in + p * gpg::Geo<1>::PN3, threadIdx.x, 4,
-                                  [dst](int x, int y, int z, float v) { dst[(z * 10 + y) * 10 + x] = v; });
-}
-
-// X0 [P*1000][8] bf16 and the per-patch scale s = max |shell potential|
-__global__ void __launch_bounds__(256) prep_input_kernel(const float *__restrict__ rho, const float *__restrict__ cube,
-                                                         __nv_bfloat16 *__restrict__ x0, float *__restrict__ scale,
-                                                         float cnst, int64_t npatch) {
-  const int64_t p = blockIdx.x;
-  if (p >= npatch) return;
+// Layer-1 input planes of one patch (one CTA): the interpolated cube (the SOR's
+// initial cube), its scale s = max |shell potential|, and per cell the channels
+// Const*rho / s (interior), phi / s (shell), interior mask
+__global__ void __launch_bounds__(256) input_kernel(const float *__restrict__ rho, const float *__restrict__ pot_in,
+                                                    __nv_bfloat16 *__restrict__ x0, float *__restrict__ scale,
+                                                    float cnst) {
+  __shared__ float cube[kCells];
   __shared__ float red[8];
+  const int64_t p = blockIdx.x;
+  gpg::interpolate<float, 1, 256>(pot_in + p * gpg::Geo<1>::PN3, threadIdx.x, 4,
+                                  [](int x, int y, int z, float v) { cube[(z * 10 + y) * 10 + x] = v; });
+  __syncthreads();
   float mx = 0.f;
   for (int v = threadIdx.x; v < kCells; v += 256) {
     const int x = v % 10, y = (v / 10) % 10, z = v / 100;
     const bool shell = x == 0 || y == 0 || z == 0 || x == 9 || y == 9 || z == 9;
-    if (shell) mx = fmaxf(mx, fabsf(cube[p * kCells + v]));
+    if (shell) mx = fmaxf(mx, fabsf(cube[v]));
   }
 #pragma unroll
   for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -106,125 +103,88 @@ __global__ void __launch_bounds__(256) prep_input_kernel(const float *__restrict
     __align__(16) __nv_bfloat16 o[8];
     const float r = shell ? 0.f : __fmul_rn(cnst, rho[p * 512 + ((z - 1) * 8 + (y - 1)) * 8 + (x - 1)]) / s;
     o[0] = __float2bfloat16_rn(r);
-    o[1] = __float2bfloat16_rn(shell ? cube[p * kCells + v] / s : 0.f);
+    o[1] = __float2bfloat16_rn(shell ? cube[v] / s : 0.f);
     o[2] = __float2bfloat16_rn(shell ? 0.f : 1.f);
 #pragma unroll
     for (int i = 3; i < 8; ++i) o[i] = __float2bfloat16_rn(0.f);
-    *reinterpret_cast<uint4 *>(x0 + (p * kCells + v) * 8) = *reinterpret_cast<const uint4 *>(o);
+    const int row = (y + 1) * gpg::net::kPlaneLine + x + 1;
+    *reinterpret_cast<uint4 *>(x0 + gpg::net::plane_at(p, z, 0, 1) + row * 8) = *reinterpret_cast<const uint4 *>(o);
   }
 }
 
-// loss partials and G4 = d loss / d y4 (channel 0 on interior cells)
-__global__ void __launch_bounds__(256) loss_grad_kernel(const float *__restrict__ y4, const float *__restrict__ target,
-                                                        const float *__restrict__ scale, __nv_bfloat16 *__restrict__ g4,
-                                                        double *__restrict__ loss_part, int64_t npatch) {
-  const int64_t M = npatch * kCells;
-  const double inv = 1.0 / double(npatch * 512);
-  double l = 0.0;
-  for (int64_t m = blockIdx.x * 256 + threadIdx.x; m < M; m += int64_t(gridDim.x) * 256) {
-    const int64_t p = m / kCells;
-    const int v = int(m - p * kCells);
-    const int x = v % 10, y = (v / 10) % 10, z = v / 100;
-    const bool interior = x > 0 && y > 0 && z > 0 && x < 9 && y < 9 && z < 9;
-    __align__(16) __nv_bfloat16 o[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) o[i] = __float2bfloat16_rn(0.f);
-    if (interior) {
-      const float t = target[p * 512 + ((z - 1) * 8 + (y - 1)) * 8 + (x - 1)] / scale[p];
-      const double d = double(y4[m * 16]) - double(t);
-      l += d * d;
-      o[0] = __float2bfloat16_rn(float(2.0 * d * inv));
+// Second stage of the gradients: parameter i = sum of the CTAs' partial sums of
+// its layer (fixed order; four threads share a parameter's partials).  Layer
+// 4's output channels 1..15 have no gradient.  The loss rides along.
+struct ReduceArgs {
+  const float *wpart[kLayers];  // [nw][27 * cin][kept channels]
+  const float *bpart[kLayers];  // [nb][32]
+  int nw[kLayers], nb[kLayers];
+  int first[kLayers + 1], weights[kLayers];  // a layer's first parameter, its number of weights
+  const double *loss_part;
+  int nloss;
+  float *grad, *loss;
+};
+
+__global__ void __launch_bounds__(256) reduce_kernel(const ReduceArgs a) {
+  __shared__ float sums[4][64];
+  const int v = threadIdx.x & 63, q = threadIdx.x >> 6;
+  constexpr int kOut4 = 16;  // output channels of layer 4, padded
+  const int i = blockIdx.x * 64 + v, total = a.first[kLayers];
+  float s = 0.f;
+  if (i < total) {
+    int l = 0;
+    while (l + 1 < kLayers && i >= a.first[l + 1]) ++l;
+    const int k = i - a.first[l], nw = a.weights[l];
+    const float *src = nullptr;
+    int64_t stride = 0;
+    int n = 0;
+    if (k >= nw) {
+      if (l < 3 || k == nw) src = a.bpart[l] + (k - nw), stride = 32, n = a.nb[l];
+    } else if (l < 3) {
+      src = a.wpart[l] + k, stride = nw, n = a.nw[l];
+    } else if (k % kOut4 == 0) {
+      src = a.wpart[3] + k / kOut4, stride = nw / kOut4, n = a.nw[3];
     }
-    uint4 *dst = reinterpret_cast<uint4 *>(g4 + m * 16);
-    dst[0] = reinterpret_cast<const uint4 *>(o)[0];
-    dst[1] = reinterpret_cast<const uint4 *>(o)[1];
-  }
-  __shared__ double red[8];
+    for (int c0 = q; c0 < n; c0 += 4 * 37) {  // 37 loads in flight (148 CTAs: all of them)
+      float x[37];
 #pragma unroll
-  for (int o = 16; o; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = l;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int w = 0; w < 8; ++w) s += red[w];
-    loss_part[blockIdx.x] = s * inv;
+      for (int c = 0; c < 37; ++c) x[c] = c0 + 4 * c < n ? src[(c0 + 4 * c) * stride] : 0.f;
+#pragma unroll
+      for (int c = 0; c < 37; ++c) s += x[c];
+    }
   }
-}
-
-// sum of the loss partials in a fixed order
-__global__ void sum_kernel(const double *p, int n, float *out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
+  sums[q][v] = s;
+  __syncthreads();
+  if (q == 0 && i < total) a.grad[i] = (sums[0][v] + sums[1][v]) + (sums[2][v] + sums[3][v]);
+  if (blockIdx.x == 0 && a.loss && threadIdx.x < 32) {
     double t = 0.0;
-    for (int i = 0; i < n; ++i) t += p[i];
-    *out = float(t);
+    for (int c = threadIdx.x; c < a.nloss; c += 32) t += a.loss_part[c];
+    t = gpg::warp_sum(t);
+    if (threadIdx.x == 0) *a.loss = float(t);
   }
 }
 
-__global__ void guess_kernel(const float *__restrict__ y4, const float *__restrict__ scale, float *__restrict__ guess,
-                             int64_t npatch) {
-  const int64_t n = npatch * 512;
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t p = i / 512;
-    const int q = int(i - p * 512), x = q % 8 + 1, y = (q / 8) % 8 + 1, z = q / 64 + 1;
-    guess[i] = y4[(p * kCells + (z * 10 + y) * 10 + x) * 16] * scale[p];
-  }
-}
-
-// bias gradient partials: part[block][n] = sum over the block's rows of g[m][n]
-template <int NOUT>
-__global__ void __launch_bounds__(256) bias_grad_kernel(const __nv_bfloat16 *__restrict__ g, float *__restrict__ part,
-                                                        int64_t M) {
-  __shared__ float red[256][NOUT + 1];
-  float acc[NOUT];
-#pragma unroll
-  for (int n = 0; n < NOUT; ++n) acc[n] = 0.f;
-  for (int64_t m = blockIdx.x * 256 + threadIdx.x; m < M; m += int64_t(gridDim.x) * 256)
-#pragma unroll
-    for (int n = 0; n < NOUT; ++n) acc[n] += __bfloat162float(g[m * NOUT + n]);
-#pragma unroll
-  for (int n = 0; n < NOUT; ++n) red[threadIdx.x][n] = acc[n];
-  __syncthreads();
-  if (threadIdx.x < NOUT) {
-    float s = 0.f;
-    for (int t = 0; t < 256; ++t) s += red[t][threadIdx.x];
-    part[blockIdx.x * NOUT + threadIdx.x] = s;
-  }
-}
-
-// grad[i] = sum_c part[c][row(i)][col(i)] for one layer's weights (+ its bias)
-__global__ void reduce_grad_kernel(const float *__restrict__ wpart, int nwpart, int wrows_stride, int kreal,
-                                   int nout, const float *__restrict__ bpart, int nbpart, float *__restrict__ grad_w,
-                                   float *__restrict__ grad_b) {
-  const int nw = kreal * nout;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nw + nout; i += gridDim.x * blockDim.x) {
-    float s = 0.f;
-    if (i < nw) {
-      for (int c = 0; c < nwpart; ++c) s += wpart[int64_t(c) * wrows_stride * nout + i];
-      grad_w[i] = s;
-    } else {
-      const int n = i - nw;
-      for (int c = 0; c < nbpart; ++c) s += bpart[c * nout + n];
-      grad_b[n] = s;
-    }
-  }
-}
-
-// pack W[27][cin][cout] (FP32) into the forward operand [KCH][cout][8] (bf16,
-// k = tap*cin + c) and, when bwd != nullptr, the backward-data operand
-// [KCH'][cin][8] with k' = tap'*cout + n and W'[tap'][n][c] = W[26-tap'][c][n]
+// pack W[27][cin][cout] (FP32) into BF16 operands:
+//   fwd  [KCH][cout][8], k = tap*cin + c (the one-kernel forward pass, layer 1)
+//   fwd3 [(dy, dx)][cin/8][dz, n][8]      (streamed kernels: three dz per MMA)
+//   bwd3 the same for the backward-data operand, W'[tap][n][c] = W[26-tap][c][n]:
+//        [(dy, dx)][cout/8][dz, c][8]
 __global__ void pack_kernel(const float *__restrict__ w, int cin, int cout, int kch_f, __nv_bfloat16 *__restrict__ fwd,
-                            int kch_b, __nv_bfloat16 *__restrict__ bwd) {
-  const int nf = kch_f * cout * 8, nb = bwd ? kch_b * cin * 8 : 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nf + nb; i += gridDim.x * blockDim.x) {
+                            __nv_bfloat16 *__restrict__ fwd3, __nv_bfloat16 *__restrict__ bwd3) {
+  const int nf = kch_f * cout * 8, n3 = fwd3 ? 27 * cin * cout : 0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nf + 2 * n3; i += gridDim.x * blockDim.x) {
     if (i < nf) {
       const int chunk = i / (cout * 8), n = (i / 8) % cout, e = i % 8;
       const int k = chunk * 8 + e, tap = k / cin, c = k % cin;
       fwd[i] = __float2bfloat16_rn(tap < 27 ? w[(tap * cin + c) * cout + n] : 0.f);
     } else {
-      const int j = i - nf;
-      const int chunk = j / (cin * 8), c = (j / 8) % cin, e = j % 8;
-      const int k = chunk * 8 + e, tap = k / cout, n = k % cout;
-      bwd[j] = __float2bfloat16_rn(tap < 27 ? w[((26 - tap) * cin + c) * cout + n] : 0.f);
+      const bool back = i >= nf + n3;
+      const int j = i - nf - (back ? n3 : 0), in = back ? cout : cin, out = back ? cin : cout;
+      const int e = j % 8, row = (j / 8) % (3 * out), chunk = j / (8 * 3 * out);
+      const int yx = chunk / (in / 8), ch = (chunk % (in / 8)) * 8 + e;  // input channel
+      const int tap = (row / out) * 9 + yx, o = row % out;               // output channel
+      const float x = back ? w[((26 - tap) * cin + o) * cout + ch] : w[(tap * cin + ch) * cout + o];
+      (back ? bwd3 : fwd3)[j] = __float2bfloat16_rn(x);
     }
   }
 }
@@ -258,9 +218,6 @@ int set_attr_once(F *fn, size_t bytes, DevOnce &st) {
   return GPG_OK;
 }
 
-// blocks of the bias-gradient and loss kernels = partial sums they leave
-constexpr int kPartials = 148;
-
 // SM count of the current device (cached per device)
 int sm_count() {
   static int n[kMaxDevices] = {};
@@ -274,40 +231,55 @@ int sm_count() {
   return n[dev];
 }
 
-template <int CIN, int NOUT, int EPI>
-int launch_conv(const ConvArgs &a, cudaStream_t s) {
+// Planes per unit: the most (fewest halo planes loaded twice) that still leaves
+// four units per SM, so that the last round of units is a small part of the
+// whole; 1 for the smallest batches.
+int unit_planes(int64_t npatch, int nz, int zmax) {
+  for (int zc = zmax; zc > 1; --zc)
+    if (nz % zc == 0 && npatch * (nz / zc) >= 4 * int64_t(sm_count())) return zc;
+  return 1;
+}
+
+// persistent CTAs: one per SM
+int unit_grid(int64_t npatch, int nz, int zc) {
+  return (int)std::min<int64_t>(npatch * (nz / zc), sm_count());
+}
+
+int launch_conv1(ConvArgs a, cudaStream_t s) {
   static DevOnce once;
-  constexpr size_t smem = gpg::net::ConvSmem<CIN, NOUT>::bytes;
-  auto fn = gpg::net::conv_fwd_kernel<CIN, NOUT, EPI>;
-  if (int rc = set_attr_once(fn, smem, once)) return rc;
-  const int64_t ntile = (a.M + 127) / 128;
-  // at most 512/32 TMEM column blocks per SM; shared memory bounds it earlier
-  const int64_t grid = std::min<int64_t>(ntile, int64_t(sm_count()) * 4);
-  if (grid <= 0) return GPG_OK;
-  fn<<<(unsigned)grid, 128, smem, s>>>(a);
+  using C = gpg::net::Conv1Cfg;
+  if (int rc = set_attr_once(gpg::net::conv1_kernel, C::bytes, once)) return rc;
+  a.zc = unit_planes(a.npatch, kEdge, kEdge);
+  gpg::net::conv1_kernel<<<(unsigned)unit_grid(a.npatch, kEdge, a.zc), C::THREADS, C::bytes, s>>>(a);
   NET_CUDA(cudaGetLastError());
   return GPG_OK;
 }
 
-template <int CIN, int NOUT>
-int wgrad_grid(int64_t M) {
-  using W = gpg::net::WgradCfg<CIN, NOUT>;
-  const int per_sm = 512 / W::COLS;
-  return (int)std::min<int64_t>((M + 127) / 128, int64_t(sm_count()) * (per_sm < 4 ? per_sm : 4));
+template <int CIN, int NOUT, int EPI>
+int launch_conv(ConvArgs a, cudaStream_t s, int *grid_out = nullptr) {
+  static DevOnce once;
+  using C = gpg::net::ConvCfg<CIN, NOUT>;
+  constexpr int nz = gpg::net::PlaneEpilogue<NOUT, EPI>::NZ;
+  auto fn = gpg::net::conv_kernel<CIN, NOUT, EPI>;
+  if (int rc = set_attr_once(fn, C::bytes, once)) return rc;
+  a.zc = unit_planes(a.npatch, nz, nz);
+  const int grid = unit_grid(a.npatch, nz, a.zc);
+  if (grid_out) *grid_out = grid;
+  fn<<<(unsigned)grid, C::THREADS, C::bytes, s>>>(a);
+  NET_CUDA(cudaGetLastError());
+  return GPG_OK;
 }
 
-template <int CIN, int NOUT>
-int launch_wgrad(const WgradArgs &a, int grid, cudaStream_t s) {
-  using W = gpg::net::WgradCfg<CIN, NOUT>;
+template <int CIN, bool LAST>
+int launch_wgrad(WgradArgs a, cudaStream_t s, int *grid_out) {
   static DevOnce once;
-  // shared memory sized so that the CTAs an SM holds never ask for more than
-  // its 512 TMEM columns in total
-  const int per_sm = 512 / W::COLS;
-  const size_t smem = std::max<size_t>(W::bytes, per_sm >= 6 ? W::bytes : (220 * 1024) / per_sm);
-  auto fn = gpg::net::conv_wgrad_kernel<CIN, NOUT>;
-  if (int rc = set_attr_once(fn, smem, once)) return rc;
-  if (grid <= 0) return GPG_OK;
-  fn<<<(unsigned)grid, 128, smem, s>>>(a);
+  using W = gpg::net::WgradCfg<CIN, LAST>;
+  auto fn = gpg::net::wgrad_kernel<CIN, LAST>;
+  if (int rc = set_attr_once(fn, W::bytes, once)) return rc;
+  a.zc = unit_planes(a.npatch, kEdge, W::ZMAX);
+  const int grid = unit_grid(a.npatch, kEdge, a.zc);
+  *grid_out = grid;
+  fn<<<(unsigned)grid, W::THREADS, W::bytes, s>>>(a);
   NET_CUDA(cudaGetLastError());
   return GPG_OK;
 }
@@ -323,9 +295,10 @@ struct gpg_net {
   int probe_polls = 0;  // test hook of the inference kernel (gpg_net_set_wait_probe)
   int64_t step = 0;
   float *params = nullptr, *grad = nullptr, *adam_m = nullptr, *adam_v = nullptr;
-  __nv_bfloat16 *wf[kLayers] = {}, *wb[kLayers] = {};
-  __nv_bfloat16 *x0 = nullptr, *act[3] = {}, *g4 = nullptr, *ga = nullptr, *gb = nullptr;
-  float *y4 = nullptr, *cube = nullptr, *scale = nullptr, *wpart = nullptr, *bpart = nullptr;
+  __nv_bfloat16 *wf[kLayers] = {}, *wf3[kLayers] = {}, *wb3[kLayers] = {};
+  // planes: input, activations (each replaced by its gradient on the way back), loss gradient
+  __nv_bfloat16 *x0 = nullptr, *act[3] = {}, *g4 = nullptr;
+  float *scale = nullptr, *wpart[kLayers] = {}, *bpart[kLayers] = {};
   double *loss_part = nullptr;
   int *err = nullptr;
 };
@@ -333,95 +306,88 @@ struct gpg_net {
 namespace {
 
 int kch_fwd(int l) { return (27 * (kCin[l] / 8) + 1) / 2 * 2; }
-int kch_bwd(int l) { return (27 * (kCout[l] / 8) + 1) / 2 * 2; }
 
 int repack(gpg_net *n, cudaStream_t s) {
   for (int l = 0; l < kLayers; ++l) {
-    pack_kernel<<<64, 256, 0, s>>>(n->params + param_offset_w(l), kCin[l], kCout[l], kch_fwd(l), n->wf[l],
-                                   kch_bwd(l), l > 0 ? n->wb[l] : nullptr);
+    pack_kernel<<<64, 256, 0, s>>>(n->params + param_offset_w(l), kCin[l], kCout[l], kch_fwd(l), n->wf[l], n->wf3[l],
+                                   n->wb3[l]);
   }
   NET_CUDA(cudaGetLastError());
   return GPG_OK;
 }
 
-int conv_forward_layer(gpg_net *n, int l, const __nv_bfloat16 *x, void *y, int64_t M, cudaStream_t s) {
-  ConvArgs a{x, n->wf[l], n->params + param_offset_b(l), y, nullptr, M, n->err};
-  switch (l) {
-    case 0: return launch_conv<8, 32, gpg::net::EPI_RELU>(a, s);
-    case 1:
-    case 2: return launch_conv<32, 32, gpg::net::EPI_RELU>(a, s);
-    default: return launch_conv<32, 16, gpg::net::EPI_LINEAR_F32>(a, s);
-  }
+ConvArgs conv_args(gpg_net *n, int64_t npatch) {
+  ConvArgs a{};
+  a.scale = n->scale;
+  a.inv = 1.0 / double(npatch * 512);
+  a.loss_part = n->loss_part;
+  a.npatch = npatch;
+  a.err = n->err;
+  return a;
 }
 
-// gradient wrt the input of layer l (> 0), masked by ReLU' of that input
-int conv_backward_data(gpg_net *n, int l, const __nv_bfloat16 *g, __nv_bfloat16 *gout, int64_t M, cudaStream_t s) {
-  ConvArgs a{g, n->wb[l], nullptr, gout, n->act[l - 1], M, n->err};
-  if (l == 3) return launch_conv<16, 32, gpg::net::EPI_MASK>(a, s);
-  return launch_conv<32, 32, gpg::net::EPI_MASK>(a, s);
-}
-
-int conv_weight_grad(gpg_net *n, int l, const __nv_bfloat16 *x, const __nv_bfloat16 *g, int64_t M, cudaStream_t s) {
-  int grid, rows;
-  WgradArgs a{x, g, n->wpart, M, n->err};
-  int rc;
-  if (l == 0) {
-    grid = wgrad_grid<8, 32>(M);
-    rows = gpg::net::WgradCfg<8, 32>::KT * 128;
-    rc = launch_wgrad<8, 32>(a, grid, s);
-  } else if (l < 3) {
-    grid = wgrad_grid<32, 32>(M);
-    rows = gpg::net::WgradCfg<32, 32>::KT * 128;
-    rc = launch_wgrad<32, 32>(a, grid, s);
-  } else {
-    grid = wgrad_grid<32, 16>(M);
-    rows = gpg::net::WgradCfg<32, 16>::KT * 128;
-    rc = launch_wgrad<32, 16>(a, grid, s);
-  }
-  if (rc) return rc;
-  const int nb = kPartials;
-  if (kCout[l] == 32)
-    bias_grad_kernel<32><<<nb, 256, 0, s>>>(g, n->bpart, M);
-  else
-    bias_grad_kernel<16><<<nb, 256, 0, s>>>(g, n->bpart, M);
-  reduce_grad_kernel<<<32, 256, 0, s>>>(n->wpart, grid, rows, 27 * kCin[l], kCout[l], n->bpart, nb,
-                                        n->grad + param_offset_w(l), n->grad + param_offset_b(l));
+// input planes and the activations of layers 1-3
+int forward_hidden(gpg_net *n, int64_t npatch, const float *rho, const float *pot_in, float cnst, cudaStream_t s) {
+  input_kernel<<<(unsigned)npatch, 256, 0, s>>>(rho, pot_in, n->x0, n->scale, cnst);
   NET_CUDA(cudaGetLastError());
-  return GPG_OK;
-}
-
-int forward_all(gpg_net *n, int64_t npatch, const float *rho, const float *pot_in, float cnst, cudaStream_t s) {
-  const int64_t M = npatch * kCells;
-  interp_cube_kernel<<<(unsigned)npatch, 128, 0, s>>>(pot_in, n->cube, npatch);
-  prep_input_kernel<<<(unsigned)npatch, 256, 0, s>>>(rho, n->cube, n->x0, n->scale, cnst, npatch);
-  NET_CUDA(cudaGetLastError());
-  const __nv_bfloat16 *x = n->x0;
+  ConvArgs a = conv_args(n, npatch);
   for (int l = 0; l < 3; ++l) {
-    if (int rc = conv_forward_layer(n, l, x, n->act[l], M, s)) return rc;
-    x = n->act[l];
+    a.x = l == 0 ? n->x0 : n->act[l - 1];
+    a.w = l == 0 ? n->wf[0] : n->wf3[l];
+    a.bias = n->params + param_offset_b(l);
+    a.y = n->act[l];
+    if (int rc = l == 0 ? launch_conv1(a, s) : launch_conv<32, 32, gpg::net::EPI_RELU>(a, s)) return rc;
   }
-  return conv_forward_layer(n, 3, x, n->y4, M, s);
+  return GPG_OK;
 }
 
+// Gradients of the batch into `grad`.  Going back, the gradient with respect to
+// a layer's input replaces the activation in place (its only readers are the
+// ReLU mask of that very value and the weight gradient, which has run).
 int gradients(gpg_net *n, int64_t npatch, const float *rho, const float *pot_in, const float *target, float cnst,
-              float *loss, cudaStream_t s) {
-  const int64_t M = npatch * kCells;
-  if (int rc = forward_all(n, npatch, rho, pot_in, cnst, s)) return rc;
-  const int nlp = kPartials;
-  loss_grad_kernel<<<nlp, 256, 0, s>>>(n->y4, target, n->scale, n->g4, n->loss_part, npatch);
-  NET_CUDA(cudaGetLastError());
-  // layer 4, then 3, 2, 1
-  if (int rc = conv_weight_grad(n, 3, n->act[2], n->g4, M, s)) return rc;
-  if (int rc = conv_backward_data(n, 3, n->g4, n->ga, M, s)) return rc;
-  if (int rc = conv_weight_grad(n, 2, n->act[1], n->ga, M, s)) return rc;
-  if (int rc = conv_backward_data(n, 2, n->ga, n->gb, M, s)) return rc;
-  if (int rc = conv_weight_grad(n, 1, n->act[0], n->gb, M, s)) return rc;
-  if (int rc = conv_backward_data(n, 1, n->gb, n->ga, M, s)) return rc;
-  if (int rc = conv_weight_grad(n, 0, n->x0, n->ga, M, s)) return rc;
-  if (loss) {
-    sum_kernel<<<1, 32, 0, s>>>(n->loss_part, nlp, loss);
-    NET_CUDA(cudaGetLastError());
+              float *grad, float *loss, cudaStream_t s) {
+  if (int rc = forward_hidden(n, npatch, rho, pot_in, cnst, s)) return rc;
+  ReduceArgs r{};
+  for (int l = 0; l < kLayers; ++l) {
+    r.first[l] = int(param_offset_w(l));
+    r.weights[l] = int(w_count(l));
   }
+  r.first[kLayers] = int(kParams);
+  r.loss_part = n->loss_part;
+  r.grad = grad;
+  r.loss = loss;
+  {
+    ConvArgs a = conv_args(n, npatch);
+    a.x = n->act[2];
+    a.w = n->wf3[3];
+    a.bias = n->params + param_offset_b(3);
+    a.y = n->g4;
+    a.target = target;
+    a.bias_part = n->bpart[3];
+    if (int rc = launch_conv<32, 16, gpg::net::EPI_LOSS>(a, s, &r.nb[3])) return rc;
+    r.nloss = r.nb[3];
+  }
+  for (int l = 3; l >= 0; --l) {
+    const __nv_bfloat16 *g = l == 3 ? n->g4 : n->act[l];
+    WgradArgs w{l == 0 ? n->x0 : n->act[l - 1], g, n->wpart[l], npatch, 0, n->err};
+    if (int rc = l == 3   ? launch_wgrad<32, true>(w, s, &r.nw[l])
+                 : l == 0 ? launch_wgrad<8, false>(w, s, &r.nw[l])
+                          : launch_wgrad<32, false>(w, s, &r.nw[l]))
+      return rc;
+    r.wpart[l] = n->wpart[l];
+    r.bpart[l] = n->bpart[l];
+    if (l == 0) break;
+    ConvArgs a = conv_args(n, npatch);
+    a.x = g;
+    a.w = n->wb3[l];
+    a.y = n->act[l - 1];
+    a.bias_part = n->bpart[l - 1];
+    if (int rc = l == 3 ? launch_conv<16, 32, gpg::net::EPI_MASK>(a, s, &r.nb[l - 1])
+                        : launch_conv<32, 32, gpg::net::EPI_MASK>(a, s, &r.nb[l - 1]))
+      return rc;
+  }
+  reduce_kernel<<<(unsigned)((kParams + 63) / 64), 256, 0, s>>>(r);
+  NET_CUDA(cudaGetLastError());
   return GPG_OK;
 }
 
@@ -432,18 +398,17 @@ void free_net(gpg_net *n) {
   cudaFree(n->adam_v);
   for (int l = 0; l < kLayers; ++l) {
     cudaFree(n->wf[l]);
-    cudaFree(n->wb[l]);
+    cudaFree(n->wf3[l]);
+    cudaFree(n->wb3[l]);
   }
   cudaFree(n->x0);
   for (auto *p : n->act) cudaFree(p);
   cudaFree(n->g4);
-  cudaFree(n->ga);
-  cudaFree(n->gb);
-  cudaFree(n->y4);
-  cudaFree(n->cube);
   cudaFree(n->scale);
-  cudaFree(n->wpart);
-  cudaFree(n->bpart);
+  for (int l = 0; l < kLayers; ++l) {
+    cudaFree(n->wpart[l]);
+    cudaFree(n->bpart[l]);
+  }
   cudaFree(n->loss_part);
   cudaFree(n->err);
 }
@@ -470,9 +435,6 @@ extern "C" int gpg_net_create(gpg_net **out, int max_batch, uint64_t seed, int d
   auto *n = new gpg_net;
   n->device = device_id;
   n->max_batch = max_batch;
-  const int64_t M = int64_t(max_batch) * kCells;
-  const int wrows = 7 * 128;  // most k rows a layer's weight gradient has
-  const int max_grid = sm_count() * 4;
   cudaError_t e = cudaSuccess;
   auto al = [&](void **p, size_t b) {
     if (e == cudaSuccess) e = cudaMalloc(p, b);
@@ -484,19 +446,22 @@ extern "C" int gpg_net_create(gpg_net **out, int max_batch, uint64_t seed, int d
   al((void **)&n->adam_v, kParams * 4);
   for (int l = 0; l < kLayers; ++l) {
     al((void **)&n->wf[l], size_t(kch_fwd(l)) * kCout[l] * 16);
-    if (l > 0) al((void **)&n->wb[l], size_t(kch_bwd(l)) * kCin[l] * 16);
+    if (l > 0) {
+      al((void **)&n->wf3[l], size_t(w_count(l)) * 2);
+      al((void **)&n->wb3[l], size_t(w_count(l)) * 2);
+    }
   }
-  al((void **)&n->x0, size_t(M) * 8 * 2);
-  for (auto &p : n->act) al((void **)&p, size_t(M) * 32 * 2);
-  al((void **)&n->g4, size_t(M) * 16 * 2);
-  al((void **)&n->ga, size_t(M) * 32 * 2);
-  al((void **)&n->gb, size_t(M) * 32 * 2);
-  al((void **)&n->y4, size_t(M) * 16 * 4);
-  al((void **)&n->cube, size_t(max_batch) * kCells * 4);
+  // zero-filled: the kernels write cells only, the planes' other rows stay zero
+  al((void **)&n->x0, size_t(max_batch) * plane_elems(8) * 2);
+  for (auto &p : n->act) al((void **)&p, size_t(max_batch) * plane_elems(32) * 2);
+  al((void **)&n->g4, size_t(max_batch) * plane_elems(16) * 2);
   al((void **)&n->scale, size_t(max_batch) * 4);
-  al((void **)&n->wpart, size_t(max_grid) * wrows * 32 * 4);
-  al((void **)&n->bpart, size_t(kPartials) * 32 * 4);
-  al((void **)&n->loss_part, kPartials * 8);
+  const size_t ctas = sm_count();  // one per SM at most
+  for (int l = 0; l < kLayers; ++l) {
+    al((void **)&n->wpart[l], ctas * 27 * kCin[l] * (l == 3 ? 1 : 32) * 4);
+    al((void **)&n->bpart[l], ctas * 32 * 4);
+  }
+  al((void **)&n->loss_part, ctas * 8);
   al((void **)&n->err, 4);
   if (e != cudaSuccess) {
     free_net(n);
@@ -621,9 +586,13 @@ extern "C" int gpg_net_predict_layers(gpg_net *n, int npatch, const float *d_rho
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   for (int64_t p0 = 0; p0 < npatch; p0 += n->max_batch) {
     const int64_t b = std::min<int64_t>(n->max_batch, npatch - p0);
-    if (int rc = forward_all(n, b, d_rho + p0 * 512, d_pot_in + p0 * 512, float(cnst), s)) return rc;
-    guess_kernel<<<296, 256, 0, s>>>(n->y4, n->scale, d_guess + p0 * 512, b);
-    NET_CUDA(cudaGetLastError());
+    if (int rc = forward_hidden(n, b, d_rho + p0 * 512, d_pot_in + p0 * 512, float(cnst), s)) return rc;
+    ConvArgs a = conv_args(n, b);
+    a.x = n->act[2];
+    a.w = n->wf3[3];
+    a.bias = n->params + param_offset_b(3);
+    a.guess = d_guess + p0 * 512;
+    if (int rc = launch_conv<32, 16, gpg::net::EPI_GUESS>(a, s)) return rc;
   }
   return GPG_OK;
 }
@@ -635,9 +604,7 @@ extern "C" int gpg_net_gradients(gpg_net *n, int npatch, const float *d_rho, con
   if (!d_rho || !d_pot_in || !d_target) return nfail(GPG_ERR_INVALID, "NULL array");
   NET_CUDA(cudaSetDevice(n->device));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (int rc = gradients(n, npatch, d_rho, d_pot_in, d_target, float(cnst), d_loss, s)) return rc;
-  if (d_grad) NET_CUDA(cudaMemcpyAsync(d_grad, n->grad, kParams * 4, cudaMemcpyDeviceToDevice, s));
-  return GPG_OK;
+  return gradients(n, npatch, d_rho, d_pot_in, d_target, float(cnst), d_grad ? d_grad : n->grad, d_loss, s);
 }
 
 namespace {
