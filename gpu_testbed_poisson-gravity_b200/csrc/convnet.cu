@@ -26,6 +26,7 @@
 using gpg::net::ConvArgs;
 using gpg::net::WgradArgs;
 using gpg::net::kCells;
+using gpg::net::KChunks;
 using gpg::net::kEdge;
 using gpg::net::plane_elems;
 
@@ -165,13 +166,13 @@ __global__ void __launch_bounds__(256) reduce_kernel(const ReduceArgs a) {
 }
 
 // pack W[27][cin][cout] (FP32) into BF16 operands:
-//   fwd  [KCH][cout][8], k = tap*cin + c (the one-kernel forward pass, layer 1)
-//   fwd3 [(dy, dx)][cin/8][dz, n][8]      (streamed kernels: three dz per MMA)
+//   fwd  [KCH][cout][8], k = tap*cin + c  (layer 1: two taps per MMA)
+//   fwd3 [(dy, dx)][cin/8][dz, n][8]      (the others: three dz per MMA)
 //   bwd3 the same for the backward-data operand, W'[tap][n][c] = W[26-tap][c][n]:
 //        [(dy, dx)][cout/8][dz, c][8]
 __global__ void pack_kernel(const float *__restrict__ w, int cin, int cout, int kch_f, __nv_bfloat16 *__restrict__ fwd,
                             __nv_bfloat16 *__restrict__ fwd3, __nv_bfloat16 *__restrict__ bwd3) {
-  const int nf = kch_f * cout * 8, n3 = fwd3 ? 27 * cin * cout : 0;
+  const int nf = fwd ? kch_f * cout * 8 : 0, n3 = fwd3 ? 27 * cin * cout : 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nf + 2 * n3; i += gridDim.x * blockDim.x) {
     if (i < nf) {
       const int chunk = i / (cout * 8), n = (i / 8) % cout, e = i % 8;
@@ -295,7 +296,7 @@ struct gpg_net {
   int probe_polls = 0;  // test hook of the inference kernel (gpg_net_set_wait_probe)
   int64_t step = 0;
   float *params = nullptr, *grad = nullptr, *adam_m = nullptr, *adam_v = nullptr;
-  __nv_bfloat16 *wf[kLayers] = {}, *wf3[kLayers] = {}, *wb3[kLayers] = {};
+  __nv_bfloat16 *wf0 = nullptr, *wf3[kLayers] = {}, *wb3[kLayers] = {};
   // planes: input, activations (each replaced by its gradient on the way back), loss gradient
   __nv_bfloat16 *x0 = nullptr, *act[3] = {}, *g4 = nullptr;
   float *scale = nullptr, *wpart[kLayers] = {}, *bpart[kLayers] = {};
@@ -305,12 +306,11 @@ struct gpg_net {
 
 namespace {
 
-int kch_fwd(int l) { return (27 * (kCin[l] / 8) + 1) / 2 * 2; }
 
 int repack(gpg_net *n, cudaStream_t s) {
   for (int l = 0; l < kLayers; ++l) {
-    pack_kernel<<<64, 256, 0, s>>>(n->params + param_offset_w(l), kCin[l], kCout[l], kch_fwd(l), n->wf[l], n->wf3[l],
-                                   n->wb3[l]);
+    pack_kernel<<<64, 256, 0, s>>>(n->params + param_offset_w(l), kCin[l], kCout[l], KChunks<kCin[0]>::KCH,
+                                   l == 0 ? n->wf0 : nullptr, n->wf3[l], n->wb3[l]);
   }
   NET_CUDA(cudaGetLastError());
   return GPG_OK;
@@ -333,7 +333,7 @@ int forward_hidden(gpg_net *n, int64_t npatch, const float *rho, const float *po
   ConvArgs a = conv_args(n, npatch);
   for (int l = 0; l < 3; ++l) {
     a.x = l == 0 ? n->x0 : n->act[l - 1];
-    a.w = l == 0 ? n->wf[0] : n->wf3[l];
+    a.w = l == 0 ? n->wf0 : n->wf3[l];
     a.bias = n->params + param_offset_b(l);
     a.y = n->act[l];
     if (int rc = l == 0 ? launch_conv1(a, s) : launch_conv<32, 32, gpg::net::EPI_RELU>(a, s)) return rc;
@@ -397,12 +397,12 @@ void free_net(gpg_net *n) {
   cudaFree(n->adam_m);
   cudaFree(n->adam_v);
   for (int l = 0; l < kLayers; ++l) {
-    cudaFree(n->wf[l]);
     cudaFree(n->wf3[l]);
     cudaFree(n->wb3[l]);
   }
   cudaFree(n->x0);
   for (auto *p : n->act) cudaFree(p);
+  cudaFree(n->wf0);
   cudaFree(n->g4);
   cudaFree(n->scale);
   for (int l = 0; l < kLayers; ++l) {
@@ -445,8 +445,9 @@ extern "C" int gpg_net_create(gpg_net **out, int max_batch, uint64_t seed, int d
   al((void **)&n->adam_m, kParams * 4);
   al((void **)&n->adam_v, kParams * 4);
   for (int l = 0; l < kLayers; ++l) {
-    al((void **)&n->wf[l], size_t(kch_fwd(l)) * kCout[l] * 16);
-    if (l > 0) {
+    if (l == 0) {
+      al((void **)&n->wf0, size_t(KChunks<kCin[0]>::KCH) * kCout[0] * 16);
+    } else {
       al((void **)&n->wf3[l], size_t(w_count(l)) * 2);
       al((void **)&n->wb3[l], size_t(w_count(l)) * 2);
     }
@@ -564,7 +565,7 @@ extern "C" int gpg_net_predict(gpg_net *n, int npatch, const float *d_rho, const
   a.pot_in = d_pot_in;
   a.guess = d_guess;
   for (int l = 0; l < kLayers; ++l) {
-    a.w[l] = n->wf[l];
+    a.w[l] = l == 0 ? n->wf0 : n->wf3[l];
     a.bias[l] = n->params + param_offset_b(l);
   }
   a.cnst = float(cnst);

@@ -2,42 +2,36 @@
 // one persistent kernel: one patch at a time per CTA, its activations resident
 // in shared memory from the interpolated input to the predicted interior.
 //
-// Layout.  A patch's 10^3 solver cube is stored as rows
-// row = (z+1)*121 + (y+1)*11 + (x+1) for cube cell (x, y, z): lines of 11
-// rows (10 cells and one zero halo column) and planes of 11 lines (10 and one
-// zero halo line), with zero halo planes before and after.  A neighbour one
-// step outside the cube in x (or y) wraps onto the halo column (line) that
-// follows, so one zero slot serves both sides.  Each row holds the cell's
-// channels as 16-byte chunks, chunk c of row r at c*1331*16 + r*16 (the
-// no-swizzle K-major core-matrix layout: 8 rows x 16 bytes contiguous;
-// consecutive chunks share their zero end planes, see kChunkRows).  Because
-// rows are contiguous, the im2col operand of tap (dz, dy, dx) for a 128-row
-// tile is the same buffer read from a start row shifted by
-// off = 121 dz + 11 dy + dx: the convolution needs no gather at all, only one
-// shared-memory descriptor per (tile, tap, K half).  The zero halo supplies the
-// "same" padding; tile rows that are not cube cells produce values that the
-// epilogue discards (their reads stay inside the kernel's shared memory).
+// Layout: the padded planes of convnet_kernels.cuh (136 rows of 16 bytes per
+// plane and 8 channels, zero halo rows), ten planes of 32 channels.  A plane's
+// window is multiplied by the weights of all three dz in one MMA (N = 96; 48 for
+// the last layer) into the accumulators of planes w+1, w, w-1, which are adjacent
+// TMEM columns.  Input plane w is read by window w alone and output plane z is
+// complete after window z+1, so every layer's output replaces its input in
+// place, and the next layer's first windows run while the last planes' epilogues
+// do.  The first layer (8 channels, a tap pair per MMA, N = 32) reads its own
+// buffer, which is filled for the next patch meanwhile.
 //
-// Roles (17 warps):
-//   * producer warp (lane 0): streams the weights in 6 units per patch (up
-//     to 28 KB: 14 taps of a 32 -> 32 layer) through a 2-slot ring with TMA bulk
-//     copies (cp.async.bulk into this CTA alone), refilling a slot once the MMAs
-//     that read it have completed (tcgen05.commit -> "empty" mbarrier).  The
-//     stream runs across layers and patches, so the next layer's weights land
-//     during the epilogue;
-//   * 16 compute warps, per patch: interpolate the coarse potential (CQUAD,
-//     same arithmetic as the SOR) into scratch, s = max |shell|, build the
-//     8-channel input rows; then per layer thread 0 issues tcgen05.mma for
-//     every tile as each unit lands (M=128, N=32 or 16, K=16, BF16 -> FP32 in
-//     TMEM; all 10 tiles of a patch accumulate at once in 320 TMEM columns,
-//     layer 4's 8 tiles in the next 128)
-//     -- it waits only for weights, never for MMAs; one mbarrier wait per
-//     unit of up to 280 MMAs -- and all 16 warps run the epilogue (tcgen05.ld; bias,
-//     ReLU, BF16) into the other activation buffer; layer 4 writes (y + b) * s
-//     of output channel 0 on the 8^3 interior straight to the guess array.
+// Roles (16 warps):
+//   * issuing warp: all MMAs in order, 10 windows per layer;
+//   * scout warp: waits for what the next window needs and passes the word on
+//     through a named barrier.  An mbarrier poll takes 100-300 cycles while MMAs
+//     saturate shared memory, longer than the queue of issued MMAs lasts;
+//   * 8 epilogue warps in two groups (planes of either parity): bias, ReLU, BF16
+//     into the planes; layer 4 writes (y + b) * s of output channel 0 on the 8^3
+//     interior straight to the guess array; accumulators go back cleared;
+//   * 4 input warps: interpolate the next patch's coarse potential (CQUAD, same
+//     arithmetic as the SOR), s = max |shell|, layer-1 planes;
+//   * loading lane: each layer's weights with one bulk copy (this CTA alone) into
+//     one of two slots, as soon as the layer before last has been multiplied.
 // Every operation and its order matches the per-layer kernels of
-// convnet_kernels.cuh (same K order per output row, same epilogue
-// arithmetic), so both paths produce the same guess.
+// convnet_kernels.cuh (same K order per output row, same epilogue arithmetic),
+// so both paths produce the same guess.
+//
+// Per patch 680 MMAs of 43 to 56 cycles each (M 128: the operand reads bound
+// them), 34.7k cycles: 0.49 ms for 4096 patches on 148 SMs.  Measured 0.65 ms;
+// 1.88 ms with one MMA of N = 32 per tap, two activation buffers and each layer's
+// epilogue after its last MMA.
 #pragma once
 
 #include <cstdint>
@@ -49,68 +43,38 @@
 namespace gpg {
 namespace net {
 
-constexpr int kLine = 11;               // rows per y line: 10 cells + 1 shared halo column
-constexpr int kPlane = 121;             // rows per z plane: 10 lines + 1 shared halo line
-constexpr int kRowCube = 133;           // row of cube cell (0,0,0) = 121 + 11 + 1
-constexpr int kRowInterior = 266;       // row of interior cell (1,1,1)
-constexpr int kMaxOffset = 133;         // largest |tap offset|
-constexpr int kTilesCube = 10;          // 128-row tiles over rows 133..1412 (cube rows end at 1330)
-constexpr int kTilesInterior = 8;       // 128-row tiles over rows 266..1289 (interior rows end at 1197)
-constexpr int kColsL4 = kTilesCube * 32;  // layer-4 accumulators follow those of layers 1-3 in TMEM
-// Chunk regions are chained 1331 rows apart: the halo plane after a chunk's
-// last cell plane (rows 1331..1451) is the halo plane before the next chunk's
-// first (rows 0..120).  Both are zero for the kernel's life, so sharing them
-// is exact.  The far corner's neighbour (+1, +1, +1) of cell (9, 9, 9) is row
-// 1463, one plane further (the next chunk's halo line and column): the chain
-// therefore ends with two zero planes after the last chunk, not one.
-constexpr int kChunkRows = 11 * kPlane;
-constexpr uint32_t kChunkBytes = kChunkRows * 16u;
-constexpr uint32_t kChainBytes = (8u * kChunkRows + 2u * kPlane) * 16u;  // buffers A and B, 4 chunks each
-// The issuing thread's wait for a weight unit slows the MMAs that follow it
-// (about 1k cycles per wait measured on B200), so units are as large as the
-// shared memory left by the activations allows: two 28 KB slots, 6 units per
-// patch (layer 1's 14 tap pairs; 14 + 13 taps of each 32 -> 32 layer; layer
-// 4's 27 taps).  While the tensor core works through one slot (>= 260 MMAs)
-// the producer refills the other.
-constexpr int kRing = 2;                // weight ring slots
-constexpr uint32_t kSlotBytes = 14 * 2048;
-__host__ __device__ constexpr int units_of_layer(int l) { return l == 0 || l == 3 ? 1 : 2; }
-__host__ __device__ constexpr int first_unit(int l) { return l == 0 ? 0 : l == 1 ? 1 : l == 2 ? 3 : 5; }
-constexpr int kUnitsPerPatch = 6;
-constexpr int kComputeThreads = 512;                // 16 warps: input, MMA issue (thread 0), epilogues
-constexpr int kInferThreads = kComputeThreads + 32; // + one producer warp for the weight ring
-constexpr int kTileGroups = kComputeThreads / 128;  // warps sharing one TMEM lane quarter
+constexpr int kInferEpi = 8, kInferIn = 4;                      // epilogue and input warps
+constexpr int kInferLoad = kInferEpi + kInferIn, kInferIssue = kInferLoad + 1, kInferScout = kInferLoad + 2;
+constexpr int kInferThreads = (kInferScout + 1) * 32;
+constexpr int kInferWindows = 4 * kEdge;                        // per patch
+constexpr uint32_t kActPlane = 4 * kPlaneChunkBytes;
+constexpr uint32_t kSlotBytes = 27 * 32 * 32 * 2;               // the largest layer's weights
 
 struct InferSmem {
-  static constexpr uint32_t buf_a = 0;
-  static constexpr uint32_t buf_b = 4 * kChunkBytes;
-  // control data in the gap between the activation chain and the ring (no
-  // descriptor read reaches it)
-  static constexpr uint32_t bias = kChainBytes;                 // 32 + 32 + 32 + 16 floats
-  static constexpr uint32_t bars = bias + 112 * 4;             // full[kRing], empty[kRing], acc
-  static constexpr uint32_t tmem_slot = bars + (2 * kRing + 1) * 8;
-  static constexpr uint32_t red = tmem_slot + 16;              // one float per compute warp
-  static constexpr uint32_t flag = red + 4 * (kComputeThreads / 32);  // abort flag
-  static constexpr uint32_t probe = flag + 8;                  // test-hook barrier (never signalled)
-  static constexpr uint32_t ring = (flag + 16 + 1023u) & ~1023u;
-  static constexpr uint32_t bytes = ring + kRing * kSlotBytes;
+  static constexpr uint32_t act = 0;                            // [10 planes][4 chunks][136 rows][8]
+  static constexpr uint32_t x0 = act + kEdge * kActPlane + kOverread;   // [12 planes][136 rows][8]
+  static constexpr uint32_t w = x0 + kPlanes * kPlaneChunkBytes + kOverread;  // two slots
+  static constexpr uint32_t bias = w + 2 * kSlotBytes;          // 32 + 32 + 32 + 16 floats
+  static constexpr uint32_t cube = bias + 112 * 4;              // interpolated cube of the input warps
+  static constexpr uint32_t scale = cube + kCells * 4;          // s of the last four patches
+  static constexpr uint32_t red = scale + 4 * 4;                // one float per input warp
+  static constexpr uint32_t bars = red + kInferIn * 4;
+  // barriers: weights full x 2, input planes full, per plane epilogue done, layer-4 accumulators cleared x 8,
+  // windows done, end, test hook
+  static constexpr int kFullW = 0, kFullX = 2, kEpi = 3, kAcc4 = kEpi + kEdge, kDone = kAcc4 + 8,
+                       kStop = kDone + kInferWindows, kProbe = kStop + 1, kBars = kProbe + 1;
+  static constexpr uint32_t tmem_slot = bars + kBars * 8;
+  static constexpr uint32_t flag = tmem_slot + 4;
+  static constexpr uint32_t bytes = flag + 4;
 };
 static_assert(InferSmem::bytes <= 232448, "shared memory per CTA");
-static_assert(InferSmem::bars % 8 == 0 && InferSmem::probe % 8 == 0, "mbarrier alignment");
-// the farthest descriptor read: buffer B, chunk 3, rows up to 133 + 128*9 + 133 + 127 = 1545
-static_assert(InferSmem::buf_b + 3 * kChunkBytes + (kRowCube + 128 * kTilesCube + kMaxOffset) * 16 <= kChainBytes,
-              "shifted tile reads stay inside the activation chain");
-static_assert(kColsL4 + kTilesInterior * 16 <= 512, "TMEM columns");
-// every read of a kept (cube) row stays inside the zero-filled chain
-static_assert(InferSmem::buf_b + 3 * kChunkBytes + (10 * kPlane + 10 * kLine + 10 + kMaxOffset + 1) * 16 <= kChainBytes,
-              "kept rows read only the zero-filled chain");
-static_assert(InferSmem::ring % 128 == 0, "ring alignment");
+static_assert(InferSmem::bars % 8 == 0 && InferSmem::w % 128 == 0 && InferSmem::x0 % 16 == 0, "alignment");
 
 struct InferArgs {
   const float *rho;              // [P][8]^3
   const float *pot_in;           // [P][8]^3 coarse potential
   float *guess;                  // [P][8]^3
-  const __nv_bfloat16 *w[4];     // packed forward operands (pack_kernel layout)
+  const __nv_bfloat16 *w[4];     // packed forward operands: layer 1 [28][32][8], then [(dy, dx)][chunk][dz, n][8]
   const float *bias[4];          // FP32 biases (32, 32, 32, 16)
   float cnst;                    // Poi_Coeff * dh^2
   int64_t npatch;
@@ -118,115 +82,45 @@ struct InferArgs {
   int probe_polls;               // > 0: thread 0 also waits that many polls on a barrier nothing signals
 };
 
-__host__ __device__ constexpr int tap_offset(int t) {
-  return (t / 9 - 1) * kPlane + ((t / 3) % 3 - 1) * kLine + (t % 3 - 1);
+__host__ __device__ constexpr uint32_t infer_weight_bytes(int l) {
+  return l == 0 ? KChunks<8>::KCH * 32 * 16 : 27u * 32 * (l == 3 ? 16 : 32) * 2;
 }
-static_assert(tap_offset(26) == kMaxOffset && tap_offset(0) == -kMaxOffset, "tap offsets");
+static_assert(infer_weight_bytes(1) == kSlotBytes && infer_weight_bytes(0) <= kSlotBytes, "weight slots");
 
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc::smem_u32(bar)), "r"(bytes)
-               : "memory");
-}
-
-// TMA bulk copy global -> this CTA's shared memory, completion on `bar`
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   tc::smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(tc::smem_u32(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ uint32_t tmem_ld1(uint32_t taddr) {
-  uint32_t r;
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr) : "memory");
-  return r;
-}
-
-// weight unit u (0..5) of the per-patch stream: its layer, first tap (tap
-// pair for layer 1), number of taps and bytes.  A tap's packed operand is
-// 2 KB (32 -> 32) or 1 KB (layer 4, and a tap pair of layer 1).
-struct Unit {
-  int layer, t0, ntap;
-  uint32_t tap_bytes;
-};
-__host__ __device__ constexpr Unit unit_info(int u) {
-  return u < 1   ? Unit{0, 0, 14, 1024u}
-         : u < 3 ? Unit{1, 14 * (u - 1), u == 1 ? 14 : 13, 2048u}
-         : u < 5 ? Unit{2, 14 * (u - 3), u == 3 ? 14 : 13, 2048u}
-                 : Unit{3, 0, 27, 1024u};
-}
-static_assert(unit_info(0).ntap == 14 && unit_info(2).t0 + unit_info(2).ntap == 27 &&
-                  unit_info(4).t0 + unit_info(4).ntap == 27 && unit_info(5).ntap == 27 &&
-                  unit_info(1).ntap * unit_info(1).tap_bytes <= kSlotBytes &&
-                  unit_info(5).ntap * unit_info(5).tap_bytes <= kSlotBytes &&
-                  first_unit(3) + units_of_layer(3) == kUnitsPerPatch,
-              "units cover every tap and fit a slot");
-__device__ __forceinline__ const unsigned char *unit_src(const InferArgs &a, int u, uint32_t &bytes) {
-  const Unit un = unit_info(u);
-  bytes = uint32_t(un.ntap) * un.tap_bytes;
-  return reinterpret_cast<const unsigned char *>(a.w[un.layer]) + uint32_t(un.t0) * un.tap_bytes;
-}
-
-// one weight unit: NT tiles x KH K-halves of M=128 MMAs into TMEM columns
-// i*NCOLS.  Descriptor steps are in units of the 16-byte start-address field.
-template <int NT, int KH, int NCOLS>
-__device__ __forceinline__ void issue_unit(uint32_t tmem, uint64_t a0, uint32_t a_step, uint64_t b0, uint32_t b_step,
-                                           uint32_t idesc, uint32_t acc_first) {
-#pragma unroll
-  for (int i = 0; i < NT; ++i)
-#pragma unroll
-    for (int jj = 0; jj < KH; ++jj)
-      tc::mma_bf16(tmem + uint32_t(i * NCOLS), a0 + uint64_t(i * 128 + jj * a_step), b0 + uint64_t(jj * b_step), idesc,
-                   jj > 0 ? 1u : acc_first);
-}
-
-// named barrier over the compute warps (the producer warp never joins)
-__device__ __forceinline__ void compute_sync() {
-  asm volatile("bar.sync 1, %0;" ::"n"(kComputeThreads) : "memory");
-}
-// the same barrier, returning whether any compute thread passed `v` true
-__device__ __forceinline__ bool compute_sync_or(bool v) {
+// Scout and issuing warp meet before every window; true when either passes
+// true (a wait gave up: both stop).
+__device__ __forceinline__ bool window_sync(bool stop) {
   uint32_t r;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.u32 p, %1, 0;\n\t"
-      "bar.red.or.pred q, 1, %2, p;\n\t"
+      "bar.red.or.pred q, 2, 64, p;\n\t"
       "selp.u32 %0, 1, 0, q;\n\t}\n"
       : "=r"(r)
-      : "r"(v ? 1u : 0u), "n"(kComputeThreads)
+      : "r"(stop ? 1u : 0u)
       : "memory");
   return r != 0;
 }
 
 __global__ void __launch_bounds__(kInferThreads, 1) net_infer_kernel(const InferArgs a) {
   using S = InferSmem;
-  extern __shared__ __align__(1024) unsigned char infer_smem[];
-  unsigned char *smem = infer_smem;
-  unsigned char *buf_a = smem + S::buf_a, *buf_b = smem + S::buf_b, *ring = smem + S::ring;
-  float *s_bias = reinterpret_cast<float *>(smem + S::bias);
-  uint64_t *full = reinterpret_cast<uint64_t *>(smem + S::bars), *empty = full + kRing, *accb = full + 2 * kRing;
+  extern __shared__ __align__(1024) unsigned char smem[];
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + S::bars);
+  uint64_t *wfull = bars + S::kFullW, *xfull = bars + S::kFullX, *epi = bars + S::kEpi, *acc4 = bars + S::kAcc4,
+           *done = bars + S::kDone, *stop = bars + S::kStop;
+  float *s_bias = reinterpret_cast<float *>(smem + S::bias), *s_scale = reinterpret_cast<float *>(smem + S::scale);
   uint32_t *s_tmem = reinterpret_cast<uint32_t *>(smem + S::tmem_slot);
-  float *s_red = reinterpret_cast<float *>(smem + S::red);
   volatile int *s_abort = reinterpret_cast<volatile int *>(smem + S::flag);
-  // scratch for the interpolated cube: buffer B chunk 1, rows 0..249 (the
-  // first 121 are chunk 0's last halo plane); zeroed again before layer 1
-  float *cube = reinterpret_cast<float *>(buf_b + kChunkBytes);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int quarter = warp & 3, group = warp >> 2;  // TMEM lanes 32*quarter.., tiles group, group+4, ...
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
 
-  // both activation buffers start at zero; the epilogues write cube rows only,
-  // so the halo rows stay zero for the kernel's life
-  for (uint32_t i = tid; i < kChainBytes / 16; i += kInferThreads)
+  // planes start at zero; only cells are ever written, so the halo rows stay zero
+  for (uint32_t i = tid; i < S::w / 16; i += kInferThreads)
     reinterpret_cast<uint4 *>(smem)[i] = make_uint4(0, 0, 0, 0);
   for (int i = tid; i < 112; i += kInferThreads)
     s_bias[i] = i < 32 ? a.bias[0][i] : i < 64 ? a.bias[1][i - 32] : i < 96 ? a.bias[2][i - 64] : a.bias[3][i - 96];
   if (tid == 0) {
-    for (int s = 0; s < kRing; ++s) {
-      tc::mbar_init(&full[s], 1);
-      tc::mbar_init(&empty[s], 1);
-    }
-    tc::mbar_init(accb, 1);
-    tc::mbar_init(reinterpret_cast<uint64_t *>(smem + S::probe), 1);
+    for (int i = 0; i < S::kBars; ++i)
+      tc::mbar_init(&bars[i], i >= S::kFullX && i < S::kDone ? 4 : 1);  // four warps fill, or hand back
     *s_abort = 0;
     tc::mbar_fence_init();
   }
@@ -236,208 +130,212 @@ __global__ void __launch_bounds__(kInferThreads, 1) net_infer_kernel(const Infer
   }
   tc::fence_proxy_async_smem();
   tc::fence_before_sync();
-  __syncthreads();  // the last barrier all 9 warps take
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = *s_tmem;
+  // accumulators: plane z of layers 1-3 at column (9 - z) * 32, of layer 4 at 320 + (8 - z) * 16
+  constexpr uint32_t kCols4 = kEdge * 32;
+  if (warp < kInferEpi) {
+    for (int h = warp >> 2; h < 28; h += kInferEpi / 4)
+      tc::tmem_zero16(tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t(h * 16));
+    tc::tmem_wait_st();
+  }
+  tc::fence_before_sync();
+  __syncthreads();
   tc::fence_after_sync();
   if (a.probe_polls > 0 && tid == 0) {
     // test hook: a bounded wait on a barrier nothing arrives on gives up
     // after probe_polls polls, records the timeout and the kernel goes on
-    tc::mbar_wait_polls(reinterpret_cast<uint64_t *>(smem + S::probe), 0, a.err, uint32_t(a.probe_polls));
+    tc::mbar_wait_polls(bars + S::kProbe, 0, a.err, uint32_t(a.probe_polls));
   }
+  const uint32_t npatch = a.npatch > blockIdx.x ? uint32_t((a.npatch - 1 - blockIdx.x) / gridDim.x + 1) : 0u;
+  auto patch_of = [&](uint32_t i) { return int64_t(blockIdx.x) + int64_t(i) * gridDim.x; };
 
-  const int64_t my_patches = a.npatch > blockIdx.x ? (a.npatch - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-  const int64_t total_units = my_patches * kUnitsPerPatch;
-
-  // ---- producer warp: stream the weight units through the ring -------------
-  if (warp == kComputeThreads / 32) {
+  if (warp == kInferLoad) {
     if (lane == 0) {
-      int64_t q_load = 0;
-      for (int64_t q = 0; q < total_units; ++q) {
-        if (*s_abort) break;
-        const int slot = int(q % kRing);
-        // the slot is free once the MMAs of unit q - kRing have completed
-        if (q >= kRing && !tc::mbar_wait(&empty[slot], uint32_t((q / kRing) - 1) & 1u, a.err)) {
+      uint32_t j = 0;
+      for (; j < 4 * npatch && !*s_abort; ++j) {
+        const uint32_t slot = j & 1u, l = j & 3u, b = j - 2;  // b: the layer that had the slot before
+        if (j >= 2 && !tc::mbar_wait(&done[(b & 3u) * kEdge + kEdge - 1], (b >> 2) & 1u, a.err)) {
           *s_abort = 1;
           break;
         }
-        uint32_t bytes;
-        const unsigned char *src = unit_src(a, int(q % kUnitsPerPatch), bytes);
-        mbar_expect_tx(&full[slot], bytes);
-        bulk_load(ring + slot * kSlotBytes, src, bytes, &full[slot]);
-        q_load = q + 1;
+        const uint32_t bytes = l == 0 ? infer_weight_bytes(0) : l == 3 ? infer_weight_bytes(3) : infer_weight_bytes(1);
+        tc::mbar_arrive_expect_tx(&wfull[slot], bytes);
+        tc::bulk_load(smem + S::w + slot * kSlotBytes, a.w[l], bytes, &wfull[slot]);
       }
-      // the last copies (one per slot) land before this warp leaves
-      for (int64_t q = q_load > kRing ? q_load - kRing : 0; q < q_load; ++q)
-        tc::mbar_wait(&full[q % kRing], uint32_t(q / kRing) & 1u, nullptr);
+      // the last copies land before the CTA leaves
+      for (uint32_t k = j > 2 ? j - 2 : 0; k < j; ++k) tc::mbar_wait(&wfull[k & 1u], (k >> 1) & 1u, nullptr);
     }
-    return;
-  }
-
-  // ---- compute warps --------------------------------------------------------
-  const uint32_t tmem = *s_tmem;
-  int64_t q_use = 0;  // thread 0: weight units consumed
-  uint32_t acc_phase = 0;
-  bool failed = false;
-
-  constexpr uint32_t IDESC32 = tc::idesc_bf16(128, 32, false, false);
-  constexpr uint32_t IDESC16 = tc::idesc_bf16(128, 16, false, false);
-  constexpr uint32_t CH = kChunkBytes;  // chunk stride (leading byte offset)
-  const uint32_t a_u32 = tc::smem_u32(buf_a), b_u32 = tc::smem_u32(buf_b), ring_u32 = tc::smem_u32(ring);
-
-  // thread 0: all MMAs of one layer and the accumulator commit; it waits only
-  // for weight units to land, never for MMAs to complete
-  auto issue_layer = [&](int layer) {
-    for (int u = first_unit(layer); u < first_unit(layer) + units_of_layer(layer); ++u) {
-      if (failed) break;
-      const int slot = int(q_use % kRing);
-      if (!tc::mbar_wait(&full[slot], uint32_t(q_use / kRing) & 1u, a.err)) {
-        failed = true;
-        *s_abort = 1;
-        break;
-      }
-      // the wait observed the copy's completion; this fence orders the
-      // asynchronous MMAs below after it (without it they may read the slot
-      // before the copy has landed)
-      tc::fence_after_sync();
-      const Unit un = unit_info(u);
-      for (int k = 0; k < un.ntap; ++k) {
-        const uint32_t wsl = ring_u32 + slot * kSlotBytes + uint32_t(k) * un.tap_bytes;
-        const int t = un.t0 + k;
-        // descriptors are built once per tap; a tile (128 rows of 16 bytes)
-        // adds 128 to the 16-byte start-address field, a K half 2 chunks
-        if (layer == 0) {  // t = tap pair (2t, 2t+1); pair 13 = tap 26 + a zero tap
-          const uint32_t lbo = t < 13 ? uint32_t(tap_offset(2 * t + 1) - tap_offset(2 * t)) * 16u : 16u;
-          issue_unit<kTilesCube, 1, 32>(tmem,
-                                        tc::smem_desc(b_u32 + uint32_t(kRowCube + tap_offset(2 * t)) * 16u, lbo, 128),
-                                        0, tc::smem_desc(wsl, 512, 128), 0, IDESC32, t > 0 ? 1u : 0u);
-        } else if (layer < 3) {
-          const uint32_t src = layer == 1 ? a_u32 : b_u32;
-          issue_unit<kTilesCube, 2, 32>(tmem, tc::smem_desc(src + uint32_t(kRowCube + tap_offset(t)) * 16u, CH, 128),
-                                        2 * CH / 16, tc::smem_desc(wsl, 512, 128), 1024 / 16, IDESC32,
-                                        t > 0 ? 1u : 0u);
-        } else {
-          issue_unit<kTilesInterior, 2, 16>(
-              tmem + kColsL4, tc::smem_desc(a_u32 + uint32_t(kRowInterior + tap_offset(t)) * 16u, CH, 128), 2 * CH / 16,
-              tc::smem_desc(wsl, 256, 128), 512 / 16, IDESC16, t > 0 ? 1u : 0u);
+  } else if (warp == kInferScout) {
+    // while the issuing warp issues a window, wait for what the next one needs
+    bool ok = true;
+    for (uint32_t i = 0; i < npatch && ok; ++i)
+      for (int l = 0; l < 4 && ok; ++l)
+        for (int w = 0; w < kEdge && ok; ++w) {
+          // one barrier per lane:
+          //  1: a layer's weights (first window)
+          //  2: layer 1: the patch's input planes; later: plane w's epilogue of the layer before
+          //  3: the accumulator opened last is cleared: plane w (layer 1: by the patch before) or w + 1
+          //  4: layer 4: its accumulator of plane w + 1, by the patch before
+          uint64_t *bar = nullptr;
+          uint32_t phase = 0;  // completions of the barrier before the one to wait for
+          if (lane == 1 && w == 0) {
+            bar = &wfull[l & 1], phase = (4 * i + l) >> 1;
+          } else if (lane == 2) {
+            if (l > 0)
+              bar = &epi[w], phase = 3 * i + l - 1;
+            else if (w == 0)
+              bar = xfull, phase = i;
+          } else if (lane == 3) {
+            const int z = l == 0 ? w : w + 1;
+            if (l < 3 && z < kEdge && (l > 0 || i > 0)) bar = &epi[z], phase = 3 * i + l - 1;
+          } else if (lane == 4) {
+            if (l == 3 && w < 8 && i > 0) bar = &acc4[w], phase = i - 1;
+          }
+          const bool got = !bar || (!*s_abort && tc::mbar_wait(bar, phase & 1u, a.err));
+          ok = __all_sync(0xffffffffu, got);
+          window_sync(!ok);
         }
+    if (!ok) *s_abort = 1;
+  } else if (warp == kInferIssue) {
+    constexpr uint32_t IDESC1 = tc::idesc_bf16(128, 32, false, false);
+    const uint32_t act = tc::smem_u32(smem + S::act), x0 = tc::smem_u32(smem + S::x0), wslot = tc::smem_u32(smem + S::w);
+    bool end = false;
+    for (uint32_t i = 0; i < npatch && !end; ++i) {
+      // layer 1: tap pairs (2j, 2j+1); 27 is a tap of zero weights
+      for (int t = 0; t < kEdge && !end; ++t) {
+        end = window_sync(false);
+        if (end) break;
+        tc::fence_after_sync();
+        const uint64_t b0 = tc::smem_desc(wslot, 32 * 16, 128);
+        auto row_of = [&](int tap) {
+          return (t + tap / 9) * kPlaneRows + kFirstRow + ((tap / 3) % 3 - 1) * kPlaneLine + tap % 3 - 1;
+        };
+#pragma unroll
+        for (int j = 0; j < 14; ++j) {
+          const int r0 = row_of(2 * j), lbo = j < 13 ? (row_of(2 * j + 1) - r0) * 16 : 16;
+          tc::mma_bf16_warp(tmem + uint32_t((kEdge - 1 - t) * 32), tc::smem_desc(x0 + r0 * 16, lbo, 128),
+                            b0 + uint64_t(j * 64), IDESC1, 1u);
+        }
+        tc::mma_commit_warp(&done[t]);
       }
-      tc::mma_commit(&empty[slot]);  // the producer may refill the slot once these MMAs are done
-      ++q_use;
-    }
-    tc::mma_commit(accb);  // also on failure, so that the other threads' wait ends
-  };
-
-  // wait for the layer's accumulators: thread 0 polls the mbarrier, the other
-  // compute threads block on the named barrier (polling from 256 threads
-  // would take shared-memory bandwidth from the tensor core's operand reads)
-  auto wait_acc = [&]() {
-    if (tid == 0 && !tc::mbar_wait(accb, acc_phase & 1u, a.err)) failed = true;
-    ++acc_phase;
-    tc::fence_before_sync();
-    failed = compute_sync_or(failed);
-    tc::fence_after_sync();
-  };
-
-  // epilogue of layers 1-3: bias + ReLU -> bf16 rows of `dst`
-  auto epilogue_relu = [&](unsigned char *dst, const float *bias) {
-    for (int i = group; i < kTilesCube; i += kTileGroups) {
-      float v[32];
-      float (&v0)[16] = *reinterpret_cast<float(*)[16]>(v);
-      float (&v1)[16] = *reinterpret_cast<float(*)[16]>(v + 16);
-      const uint32_t ta = tmem + (uint32_t(32 * quarter) << 16) + uint32_t(i * 32);
-      tc::tmem_ld16(ta, v0);
-      tc::tmem_ld16(ta + 16, v1);
-      tc::tmem_wait_ld();
-      const int row = kRowCube + 128 * i + 32 * quarter + lane;
-      const int z = row / kPlane, r2 = row - z * kPlane, y = r2 / kLine, x = r2 - y * kLine;
-      if (x >= 1 && y >= 1 && z >= 1 && z <= 10) {  // x, y <= 10 always
+      for (int l = 1; l < 4 && !end; ++l) {
+        const uint32_t nout = l == 3 ? 16 : 32;
+        const uint64_t b0 = tc::smem_desc(wslot + (l & 1) * kSlotBytes, 3 * nout * 16, 128);
+        const int zmin = l == 3 ? 1 : 0, zmax = l == 3 ? 8 : 9;
+        for (int w = 0; w < kEdge && !end; ++w) {
+          end = window_sync(false);
+          if (end) break;
+          tc::fence_after_sync();
+          const int hi = w + 1 < zmax ? w + 1 : zmax, lo = w - 1 > zmin ? w - 1 : zmin;
+          const uint32_t d = tmem + (l == 3 ? kCols4 + uint32_t(8 - hi) * 16 : uint32_t(9 - hi) * 32);
+          const uint32_t idesc = tc::idesc_bf16(128, 0, false, false) | (uint32_t(hi - lo + 1) * (nout / 8)) << 17;
+          const uint64_t a0 = tc::smem_desc(act + w * kActPlane, kPlaneChunkBytes, 128);
+          const uint64_t b = b0 + uint64_t((w - hi + 1) * nout);  // dz = w - z, from -1
+          const uint32_t bstep = 2 * 3 * nout;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          __align__(16) __nv_bfloat16 o[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) o[e] = __float2bfloat16_rn(fmaxf(v[8 * c + e] + bias[8 * c + e], 0.f));
-          *reinterpret_cast<uint4 *>(dst + c * CH + row * 16) = *reinterpret_cast<const uint4 *>(o);
+          for (int q = 0; q < 18; ++q) {
+            const int yx = q / 2, h = q % 2, off = kFirstRow + (yx / 3 - 1) * kPlaneLine + yx % 3 - 1 + 2 * h * kPlaneRows;
+            tc::mma_bf16_warp(d, a0 + uint64_t(off), b + uint64_t(q * bstep), idesc, 1u);
+          }
+          tc::mma_commit_warp(&done[l * kEdge + w]);
         }
       }
     }
-  };
-
-  auto end_phase = [&]() -> bool {  // smem writes -> tensor core; true when any thread failed
-    tc::fence_proxy_async_smem();
-    tc::fence_before_sync();
-    const bool stop = compute_sync_or(failed);
-    tc::fence_after_sync();
-    return stop;
-  };
-
-  for (int64_t p = blockIdx.x; p < a.npatch; p += gridDim.x) {
-    // ---- input rows (layer-1 operand, buffer B chunk 0) -------------------
-    interpolate<float, 1, kComputeThreads>(a.pot_in + p * Geo<1>::PN3, tid, 4,
+    tc::mma_commit_warp(stop);
+    tc::mbar_wait(stop, 0, nullptr);  // the MMAs have ended
+  } else if (warp >= kInferEpi) {
+    // ---- input planes, one patch ahead ---------------------------------------
+    const int t = tid - kInferEpi * 32;
+    float *cube = reinterpret_cast<float *>(smem + S::cube), *red = reinterpret_cast<float *>(smem + S::red);
+    auto sync = []() { asm volatile("bar.sync 1, %0;" ::"n"(kInferIn * 32) : "memory"); };
+    bool ok = true;
+    for (uint32_t i = 0; i < npatch; ++i) {
+      const int64_t p = patch_of(i);
+      sync();  // the previous patch's cube is read
+      interpolate<float, 1, kInferIn * 32>(a.pot_in + p * Geo<1>::PN3, t, 4,
                                            [cube](int x, int y, int z, float v) { cube[(z * 10 + y) * 10 + x] = v; });
-    compute_sync();
-    float mx = 0.f;
-    for (int v = tid; v < kCells; v += kComputeThreads) {
-      const int x = v % 10, y = (v / 10) % 10, z = v / 100;
-      if (x == 0 || y == 0 || z == 0 || x == 9 || y == 9 || z == 9) mx = fmaxf(mx, fabsf(cube[v]));
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) s_red[warp] = mx;
-    compute_sync();
-    float s = s_red[0];
-    for (int w = 1; w < kComputeThreads / 32; ++w) s = fmaxf(s, s_red[w]);
-    if (!(s > 0.f)) s = 1.f;
-    for (int v = tid; v < kCells; v += kComputeThreads) {
-      const int x = v % 10, y = (v / 10) % 10, z = v / 100;
-      const bool shell = x == 0 || y == 0 || z == 0 || x == 9 || y == 9 || z == 9;
-      __align__(16) __nv_bfloat16 o[8];
-      const float r = shell ? 0.f : __fmul_rn(a.cnst, a.rho[p * 512 + ((z - 1) * 8 + (y - 1)) * 8 + (x - 1)]) / s;
-      o[0] = __float2bfloat16_rn(r);
-      o[1] = __float2bfloat16_rn(shell ? cube[v] / s : 0.f);
-      o[2] = __float2bfloat16_rn(shell ? 0.f : 1.f);
-#pragma unroll
-      for (int i = 3; i < 8; ++i) o[i] = __float2bfloat16_rn(0.f);
-      const int row = (z + 1) * kPlane + (y + 1) * kLine + (x + 1);
-      *reinterpret_cast<uint4 *>(buf_b + row * 16) = *reinterpret_cast<const uint4 *>(o);
-    }
-    compute_sync();
-    for (int i = tid; i < kCells / 4; i += kComputeThreads) reinterpret_cast<uint4 *>(cube)[i] = make_uint4(0, 0, 0, 0);
-    if (end_phase()) break;
-
-    // ---- layers 1-3 -------------------------------------------------------
-    unsigned char *dst[3] = {buf_a, buf_b, buf_a};
-    bool stop = false;
-    for (int l = 0; l < 3 && !stop; ++l) {
-      if (warp == 0) {
-        if (lane == 0) issue_layer(l);
-        __syncwarp();
+      sync();
+      float mx = 0.f;
+      for (int v = t; v < kCells; v += kInferIn * 32) {
+        const int x = v % 10, y = (v / 10) % 10, z = v / 100;
+        if (x == 0 || y == 0 || z == 0 || x == 9 || y == 9 || z == 9) mx = fmaxf(mx, fabsf(cube[v]));
       }
-      wait_acc();
-      epilogue_relu(dst[l], s_bias + 32 * l);
-      stop = end_phase();
-    }
-    if (stop) break;
-
-    // ---- layer 4: channel 0 on the interior -> guess -----------------------
-    if (warp == 0) {
-      if (lane == 0) issue_layer(3);
+#pragma unroll
+      for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      if (lane == 0) red[warp - kInferEpi] = mx;
+      sync();
+      float s = red[0];
+      for (int w = 1; w < kInferIn; ++w) s = fmaxf(s, red[w]);
+      if (!(s > 0.f)) s = 1.f;
+      if (t == 0) s_scale[i & 3u] = s;
+      // layer 1 of the patch before has read the planes
+      int got = 1;
+      if (lane == 0 && i > 0) got = !*s_abort && tc::mbar_wait(&done[kEdge - 1], (i - 1) & 1u, a.err);
+      if (!__shfl_sync(0xffffffffu, got, 0)) ok = false;
+      for (int v = t; ok && v < kCells; v += kInferIn * 32) {
+        const int x = v % 10, y = (v / 10) % 10, z = v / 100;
+        const bool shell = x == 0 || y == 0 || z == 0 || x == 9 || y == 9 || z == 9;
+        __align__(16) __nv_bfloat16 o[8];
+        const float r = shell ? 0.f : __fmul_rn(a.cnst, a.rho[p * 512 + ((z - 1) * 8 + (y - 1)) * 8 + (x - 1)]) / s;
+        o[0] = __float2bfloat16_rn(r);
+        o[1] = __float2bfloat16_rn(shell ? cube[v] / s : 0.f);
+        o[2] = __float2bfloat16_rn(shell ? 0.f : 1.f);
+#pragma unroll
+        for (int e = 3; e < 8; ++e) o[e] = __float2bfloat16_rn(0.f);
+        const int row = (z + 1) * kPlaneRows + (y + 1) * kPlaneLine + x + 1;
+        *reinterpret_cast<uint4 *>(smem + S::x0 + row * 16) = *reinterpret_cast<const uint4 *>(o);
+      }
+      tc::fence_proxy_async_smem();
       __syncwarp();
+      if (lane == 0) tc::mbar_arrive(xfull);
     }
-    wait_acc();
-    for (int i = group; i < kTilesInterior; i += kTileGroups) {
-      const float y4 =
-          __uint_as_float(tmem_ld1(tmem + (uint32_t(32 * quarter) << 16) + uint32_t(kColsL4 + i * 16)));
-      tc::tmem_wait_ld();
-      const int row = kRowInterior + 128 * i + 32 * quarter + lane;
-      const int z = row / kPlane, r2 = row - z * kPlane, y = r2 / kLine, x = r2 - y * kLine;
-      if (x >= 2 && x <= 9 && y >= 2 && y <= 9 && z >= 2 && z <= 9)
-        a.guess[p * 512 + ((z - 2) * 8 + (y - 2)) * 8 + (x - 2)] = (y4 + s_bias[96]) * s;
+    if (!ok) *s_abort = 1;
+  } else {
+    // ---- epilogues ------------------------------------------------------------
+    const int group = warp >> 2;
+    const uint32_t lanes = tmem + (uint32_t((warp & 3) * 32) << 16);
+    const int r = kFirstRow + (tid & 127), cy = r / kPlaneLine - 1, cx = r - (cy + 1) * kPlaneLine - 1;
+    const bool cell = cx >= 0 && r <= kLastRow;
+    const bool inner = cell && cx >= 1 && cx <= 8 && cy >= 1 && cy <= 8;
+    bool ok = true;
+    for (uint32_t i = 0; i < npatch && ok; ++i) {
+      for (int l = 0; l < 3 && ok; ++l) {
+        const float *bias = s_bias + 32 * l;
+        for (int z = group; z < kEdge && ok; z += kInferEpi / 4) {
+          float acc[32];
+          const int w = l == 0 || z == kEdge - 1 ? z : z + 1;  // the plane's last window
+          ok = take_accumulator<32, true, false>(&done[l * kEdge + w], i & 1u, nullptr, lanes + (kEdge - 1 - z) * 32,
+                                                 s_abort, a.err, lane, acc);
+          if (ok && cell) {
+            unsigned char *dst = smem + S::act + z * kActPlane + r * 16;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              __align__(16) __nv_bfloat16 o[8];
+#pragma unroll
+              for (int e = 0; e < 8; ++e) o[e] = __float2bfloat16_rn(fmaxf(acc[8 * c + e] + bias[8 * c + e], 0.f));
+              *reinterpret_cast<uint4 *>(dst + c * kPlaneChunkBytes) = *reinterpret_cast<const uint4 *>(o);
+            }
+          }
+          tc::fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(&epi[z]);
+        }
+      }
+      const int64_t p = patch_of(i);
+      const float s = s_scale[i & 3u];
+      for (int z = 1 + group; z < kEdge - 1 && ok; z += kInferEpi / 4) {
+        float acc[16];
+        ok = take_accumulator<16, true, true>(&done[3 * kEdge + z + 1], i & 1u, &acc4[z - 1], lanes + kCols4 + (8 - z) * 16,
+                                              s_abort, a.err, lane, acc);
+        if (ok && inner) a.guess[p * 512 + ((z - 1) * 8 + (cy - 1)) * 8 + (cx - 1)] = (acc[0] + s_bias[96]) * s;
+      }
     }
-    if (end_phase()) break;
+    if (!ok) *s_abort = 1;
   }
-  if (failed) *s_abort = 1;
-
   tc::fence_before_sync();
-  compute_sync();
+  __syncthreads();
   if (warp == 0) {
     tc::fence_after_sync();
     tc::tmem_dealloc(tmem, 512);

@@ -206,8 +206,9 @@ struct PlaneEpilogue {
   }
 };
 
-// wait for an accumulator (one lane polls), read it, hand it back (ZERO: cleared)
-template <int NOUT, bool ZERO>
+// wait for an accumulator (one lane polls), read it, clear it (ZERO), hand it
+// back (ARRIVE; otherwise a later arrival of the caller does)
+template <int NOUT, bool ZERO, bool ARRIVE = true>
 __device__ __forceinline__ bool take_accumulator(uint64_t *full, uint32_t parity, uint64_t *empty, uint32_t taddr,
                                                  volatile int *s_abort, int *err, int lane, float (&acc)[NOUT]) {
   int got = 1;
@@ -224,8 +225,10 @@ __device__ __forceinline__ bool take_accumulator(uint64_t *full, uint32_t parity
     tc::tmem_wait_st();
   }
   tc::fence_before_sync();
-  __syncwarp();
-  if (lane == 0) tc::mbar_arrive(empty);
+  if (ARRIVE) {
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(empty);
+  }
   return true;
 }
 
