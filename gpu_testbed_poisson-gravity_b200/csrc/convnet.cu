@@ -77,11 +77,11 @@ constexpr int64_t kParams = param_offset_w(kLayers);
 // Const*rho / s (interior), phi / s (shell), interior mask
 __global__ void __launch_bounds__(256) input_kernel(const float *__restrict__ rho, const float *__restrict__ pot_in,
                                                     __nv_bfloat16 *__restrict__ x0, float *__restrict__ scale,
-                                                    float cnst) {
+                                                    float cnst, float neg_zero) {
   __shared__ float cube[kCells];
   __shared__ float red[8];
   const int64_t p = blockIdx.x;
-  gpg::interpolate<float, 1, 256>(pot_in + p * gpg::Geo<1>::PN3, threadIdx.x, 4,
+  gpg::interpolate<float, 1, 256>(pot_in + p * gpg::Geo<1>::PN3, threadIdx.x, 4, neg_zero,
                                   [](int x, int y, int z, float v) { cube[(z * 10 + y) * 10 + x] = v; });
   __syncthreads();
   float mx = 0.f;
@@ -328,7 +328,7 @@ ConvArgs conv_args(gpg_net *n, int64_t npatch) {
 
 // input planes and the activations of layers 1-3
 int forward_hidden(gpg_net *n, int64_t npatch, const float *rho, const float *pot_in, float cnst, cudaStream_t s) {
-  input_kernel<<<(unsigned)npatch, 256, 0, s>>>(rho, pot_in, n->x0, n->scale, cnst);
+  input_kernel<<<(unsigned)npatch, 256, 0, s>>>(rho, pot_in, n->x0, n->scale, cnst, -0.f);
   NET_CUDA(cudaGetLastError());
   ConvArgs a = conv_args(n, npatch);
   for (int l = 0; l < 3; ++l) {
@@ -569,6 +569,7 @@ extern "C" int gpg_net_predict(gpg_net *n, int npatch, const float *d_rho, const
     a.bias[l] = n->params + param_offset_b(l);
   }
   a.cnst = float(cnst);
+  a.neg_zero = -0.f;
   a.npatch = npatch;
   a.probe_polls = n->probe_polls;
   a.err = n->err;

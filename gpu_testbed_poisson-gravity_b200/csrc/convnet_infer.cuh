@@ -77,6 +77,7 @@ struct InferArgs {
   const __nv_bfloat16 *w[4];     // packed forward operands: layer 1 [28][32][8], then [(dy, dx)][chunk][dz, n][8]
   const float *bias[4];          // FP32 biases (32, 32, 32, 16)
   float cnst;                    // Poi_Coeff * dh^2
+  float neg_zero;                // as in SolveArgs
   int64_t npatch;
   int *err;
   int probe_polls;               // > 0: thread 0 also waits that many polls on a barrier nothing signals
@@ -254,7 +255,7 @@ __global__ void __launch_bounds__(kInferThreads, 1) net_infer_kernel(const Infer
     for (uint32_t i = 0; i < npatch; ++i) {
       const int64_t p = patch_of(i);
       sync();  // the previous patch's cube is read
-      interpolate<float, 1, kInferIn * 32>(a.pot_in + p * Geo<1>::PN3, t, 4,
+      interpolate<float, 1, kInferIn * 32>(a.pot_in + p * Geo<1>::PN3, t, 4, a.neg_zero,
                                            [cube](int x, int y, int z, float v) { cube[(z * 10 + y) * 10 + x] = v; });
       sync();
       float mx = 0.f;

@@ -114,12 +114,11 @@ constexpr int kSorVariantRows[kSorVariants] = {1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 2, 
 constexpr bool kSorVariantStaged[kSorVariants] = {false, false, false, false, false, false, false, false, false,
                                                   false, false, false, false, false, true,  true,  true};
 constexpr int kSorDefault[2][6] = {
-    // ghost:  -  1  2  3  4  5       (autotune.py on B200, 4096 patches, reference parameters)
-    // FP32 with two heights per packed register pair, us per launch, the best
-    // of this kernel against the best scalar one: g1 36.9 / 36.8, g2 58.9 / 65.9,
-    // g3 106.9 / 115.2, g4 152.6 / 168.0, g5 202.5 / 231.3
+    // ghost:  -  1  2  3  4  5       (autotune.py on B200, 4096 patches, reference parameters;
+    //   FP32 ghost 4: the whole column 138 us per launch, the split one 152; FP64 ghost 1
+    //   height by height 105.4 us, phased 106.3, ghost 3 530 and 533, with gravity 548 and 554)
     {0, 11, 10, 10, 13, 11},   // float
-    {0, 11, 13, 11, 10, 14},   // double
+    {0, 10, 13, 10, 10, 14},   // double
 };
 // atomic: gpg_set_sor_variant may run on one host thread while another launches
 std::atomic<int> g_sor_variant[2][6] = {
@@ -133,12 +132,12 @@ std::atomic<bool> g_sor_pinned[2][6] = {};
 // short of teams, and other layouts finish each patch sooner: those that split
 // each pair column between two lanes (twice the threads per patch), and for
 // FP64 ghost 4 the staged one.  Measured on B200 at 64-4096 patches per launch
-// (autotune.py --sizes, reference parameters), the variant below wins up to
-// max_npatch patches: FP32 ghost 1 at 256 patches 16.5 -> 11.3 us per launch,
-// at 1024 16.5 -> 14.6, ghost 2 at 256 14.5 -> 12.4, ghost 4 at 256 22.3 ->
-// 20.6; FP32 ghost 3 and 5 run the large-launch layout at every size (ghost 3
-// at 1024: 35.1, the one-row layout 39.3).  FP64 ghost 2 at 256 53.6 -> 39.1,
-// ghost 4 at 64 72.7 -> 59.6.  FP64 ghost 5 keeps the
+// (autotune.py --sizes, reference parameters, gravity), the variant below wins
+// up to max_npatch patches: FP32 ghost 1 at 256 patches 16.5 -> 12.4 us per
+// launch, ghost 2 16.0 -> 12.5, ghost 3 18.6 -> 16.6; FP32 ghost 5 runs the
+// large-launch layout at every size, ghost 4 the split column up to 1024 (45.6
+// us; the whole one 45.8, at 256 patches 20.6 and 22.7).  FP64 ghost 2 at 256
+// 53.6 -> 39.1, ghost 4 at 64 72.7 -> 59.6.  FP64 ghost 5 keeps the
 // unstaged v11 up to 1024 patches: the staged kernel hands patches out at a
 // fixed stride, and 1024 patches over its 296 teams leave some teams a fourth
 // patch (333 vs 360 us; through the CUAPI path, 4 streams of 1024 patches,
@@ -148,7 +147,7 @@ struct SorSmall {
 };
 constexpr SorSmall kSorSmall[2][6] = {
     // ghost:  -       1          2          3         4          5
-    {{0, 0}, {2048, 7}, {512, 6}, {0, 0}, {1024, 11}, {0, 0}},       // float
+    {{0, 0}, {2048, 7}, {512, 6}, {512, 7}, {1024, 11}, {0, 0}},     // float
     {{0, 0}, {256, 8}, {256, 7}, {0, 0}, {256, 14}, {1024, 11}},     // double
 };
 std::once_flag g_tune_once;

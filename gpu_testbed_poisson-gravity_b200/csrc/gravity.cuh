@@ -8,45 +8,145 @@
 // The density component is read, never written.
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace gpg {
 
-// `phi(i, j, k)` returns the potential at patch-cell offset (i, j, k), which
-// ranges over [-2, 10) (x fastest).  flu points at one patch [5][8][8][8].
+// One cell: phi(i, j, k) returns the potential at patch-cell offset (i, j, k),
+// which ranges over [-2, 10) (x fastest); q = rho, px, py, pz, E, updated.
+template <typename T, typename Phi>
+__device__ __forceinline__ void gravity_cell(int i, int j, int k, T gra_const, int p5, Phi phi, T (&q)[5]) {
+  const T c8 = T(8);
+  T ax, ay, az;
+  if (p5) {
+    ax = mul(gra_const, sub(add(add(-phi(i + 2, j, k), phi(i - 2, j, k)), mul(c8, phi(i + 1, j, k))),
+                            mul(c8, phi(i - 1, j, k))));
+    ay = mul(gra_const, sub(add(add(-phi(i, j + 2, k), phi(i, j - 2, k)), mul(c8, phi(i, j + 1, k))),
+                            mul(c8, phi(i, j - 1, k))));
+    az = mul(gra_const, sub(add(add(-phi(i, j, k + 2), phi(i, j, k - 2)), mul(c8, phi(i, j, k + 1))),
+                            mul(c8, phi(i, j, k - 1))));
+  } else {
+    ax = mul(gra_const, sub(phi(i + 1, j, k), phi(i - 1, j, k)));
+    ay = mul(gra_const, sub(phi(i, j + 1, k), phi(i, j - 1, k)));
+    az = mul(gra_const, sub(phi(i, j, k + 1), phi(i, j, k - 1)));
+  }
+  const T temp = divide(T(0.5), q[0]);
+  const T eint = sub(q[4], mul(temp, add(add(mul(q[1], q[1]), mul(q[2], q[2])), mul(q[3], q[3]))));
+  q[1] = sub(q[1], mul(q[0], ax));
+  q[2] = sub(q[2], mul(q[0], ay));
+  q[3] = sub(q[3], mul(q[0], az));
+  q[4] = add(eint, mul(temp, add(add(mul(q[1], q[1]), mul(q[2], q[2])), mul(q[3], q[3]))));
+}
+
+// Runs of 16 bytes (4 FP32 or 2 FP64 cells along x) of the patch's fluid, one
+// per thread and step: 128 FP32 runs instead of 512 cells, so that a team of 96
+// threads waits for two rounds of loads and not six.  flu points at one patch
+// [5][8][8][8]; a pointer off the 16-byte alignment takes the values one by one.
+template <typename T>
+struct FluidRun {
+  static constexpr int W = 16 / sizeof(T), RUNS = 512 / W;
+  T q[5][W];  // component, cell
+  __device__ __forceinline__ void load(const T *flu, int run, bool aligned) {
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+      const T *src = flu + c * 512 + run * W;
+      if (aligned) {
+        *reinterpret_cast<uint4 *>(q[c]) = *reinterpret_cast<const uint4 *>(src);
+      } else {
+#pragma unroll
+        for (int e = 0; e < W; ++e) q[c][e] = src[e];
+      }
+    }
+  }
+  __device__ __forceinline__ void store(T *flu, int run, bool aligned) const {
+#pragma unroll
+    for (int c = 1; c < 5; ++c) {  // the density is read only
+      T *dst = flu + c * 512 + run * W;
+      if (aligned) {
+        *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(q[c]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < W; ++e) dst[e] = q[c][e];
+      }
+    }
+  }
+  template <typename Phi>
+  __device__ __forceinline__ void update(int run, T gra_const, int p5, Phi phi) {
+    const int c0 = run * W;
+#pragma unroll
+    for (int e = 0; e < W; ++e) {
+      T cell[5] = {q[0][e], q[1][e], q[2][e], q[3][e], q[4][e]};
+      gravity_cell((c0 & 7) + e, (c0 >> 3) & 7, c0 >> 6, gra_const, p5, phi, cell);
+#pragma unroll
+      for (int c = 1; c < 5; ++c) q[c][e] = cell[c];
+    }
+  }
+};
+
+__device__ __forceinline__ bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 template <typename T, int NT, typename Phi>
 __device__ __forceinline__ void gravity_patch(T *__restrict__ flu, int tid, T gra_const, int p5,
                                               Phi phi) {
-  constexpr int PS3 = 512;
-  const T c8 = T(8);
-  for (int c = tid; c < PS3; c += NT) {
-    const int i = c & 7, j = (c >> 3) & 7, k = c >> 6;
-    T ax, ay, az;
-    if (p5) {
-      ax = mul(gra_const, sub(add(add(-phi(i + 2, j, k), phi(i - 2, j, k)), mul(c8, phi(i + 1, j, k))),
-                              mul(c8, phi(i - 1, j, k))));
-      ay = mul(gra_const, sub(add(add(-phi(i, j + 2, k), phi(i, j - 2, k)), mul(c8, phi(i, j + 1, k))),
-                              mul(c8, phi(i, j - 1, k))));
-      az = mul(gra_const, sub(add(add(-phi(i, j, k + 2), phi(i, j, k - 2)), mul(c8, phi(i, j, k + 1))),
-                              mul(c8, phi(i, j, k - 1))));
-    } else {
-      ax = mul(gra_const, sub(phi(i + 1, j, k), phi(i - 1, j, k)));
-      ay = mul(gra_const, sub(phi(i, j + 1, k), phi(i, j - 1, k)));
-      az = mul(gra_const, sub(phi(i, j, k + 1), phi(i, j, k - 1)));
-    }
-    const T rho = flu[c];
-    T px = flu[PS3 + c], py = flu[2 * PS3 + c], pz = flu[3 * PS3 + c];
-    const T e = flu[4 * PS3 + c];
-    const T temp = divide(T(0.5), rho);
-    const T eint = sub(e, mul(temp, add(add(mul(px, px), mul(py, py)), mul(pz, pz))));
-    px = sub(px, mul(rho, ax));
-    py = sub(py, mul(rho, ay));
-    pz = sub(pz, mul(rho, az));
-    flu[PS3 + c] = px;
-    flu[2 * PS3 + c] = py;
-    flu[3 * PS3 + c] = pz;
-    flu[4 * PS3 + c] = add(eint, mul(temp, add(add(mul(px, px), mul(py, py)), mul(pz, pz))));
+  const bool al = aligned16(flu);
+  for (int run = tid; run < FluidRun<T>::RUNS; run += NT) {
+    FluidRun<T> f;
+    f.load(flu, run, al);
+    f.update(run, gra_const, p5, phi);
+    f.store(flu, run, al);
   }
+}
+
+// What every solver kernel leaves of a patch: the GRA_NXT^3 window of the solved
+// cube (CPU_PoissonSolver_SOR.cpp:305-311) and, with gra_acc, the updated fluid.
+// cube(x, y, z) reads the solver's cube.  The first fluid loads are under way
+// while the window is written.
+template <typename T, int G, int NT, typename Cube>
+__device__ __forceinline__ void patch_output(const SolveArgs<T> &a, int64_t P, int tid, Cube cube) {
+  T *flu = a.flu + P * 5 * 512;
+  const bool al = aligned16(flu);
+  FluidRun<T> f;
+  if (a.gra_acc && tid < FluidRun<T>::RUNS) f.load(flu, tid, al);
+  // (edge GN a compile-time constant per GRA_GHOST_SIZE: the index split is
+  // then multiply-shift, not division)
+  auto window = [&](auto gg) {
+    constexpr int GG = decltype(gg)::value, GN = 8 + 2 * GG, shift = G - GG, GN3 = GN * GN * GN;
+    T *dst = a.pot_out + P * GN3;
+    for (int t = tid; t < GN3; t += NT) {
+      const int i = t % GN, j = (t / GN) % GN, k = t / (GN * GN);
+      dst[t] = cube(i + shift, j + shift, k + shift);
+    }
+  };
+  if (a.gra_ghost == 0)
+    window(std::integral_constant<int, 0>{});
+  else if (a.gra_ghost == 1)
+    window(std::integral_constant<int, 1>{});
+  else
+    window(std::integral_constant<int, 2>{});
+  // fused gravity update (CPU_GravitySolver.cpp:34-79)
+  if (a.gra_acc) {
+    auto phi = [&](int i, int j, int k) { return cube(i + G, j + G, k + G); };
+    for (int run = tid; run < FluidRun<T>::RUNS; run += NT) {
+      if (run >= NT) f.load(flu, run, al);
+      f.update(run, a.gra_const, a.p5, phi);
+      f.store(flu, run, al);
+    }
+  }
+}
+
+// Lines of a patch's density and fluid into L2: needed only once the cube is
+// interpolated, and at the end.
+template <typename T, int G, int NT>
+__device__ __forceinline__ void prefetch_patch(const SolveArgs<T> &a, int64_t P, int tid) {
+  auto lines = [tid](const void *p, int bytes) {
+    for (int o = tid * 128; o < bytes; o += NT * 128)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const char *>(p) + o));
+  };
+  using g = Geo<G>;
+  lines(a.rho + P * g::RHO3, g::RHO3 * int(sizeof(T)));
+  if (a.gra_acc) lines(a.flu + P * 5 * 512, 5 * 512 * int(sizeof(T)));
 }
 
 // Gravity alone (Poisson off): the potential comes from pot_out

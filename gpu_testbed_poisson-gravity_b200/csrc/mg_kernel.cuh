@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(NT) mg_kernel(const SolveArgs<T> a) {
 
   // level-0 solution = interpolated cube; rhs0 = Poi_Coeff * rho; def boundaries 0
   for (int t = tid; t < LV::total; t += NT) s_def[t] = T(0);
-  interpolate<T, G, NT>(a.pot_in + P * g::PN3, tid, a.int_scheme,
+  interpolate<T, G, NT>(a.pot_in + P * g::PN3, tid, a.int_scheme, a.neg_zero,
                         [s_sol](int x, int y, int z, T v) { s_sol[(z * N + y) * N + x] = v; });
   {
     const T *rho = a.rho + P * g::RHO3;

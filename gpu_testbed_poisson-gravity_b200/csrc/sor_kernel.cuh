@@ -42,6 +42,7 @@
 #include "common.cuh"
 #include "gravity.cuh"
 #include "interp.cuh"
+#include "packed.cuh"
 #include "tc_common.cuh"
 
 namespace gpg {
@@ -138,6 +139,37 @@ struct SorLane {
   bool left_even;  // colour-c cell on the left of the pair iff (zz + c) even
                    // (Y = 2: of the lane's second, even row)
 };
+
+// Thread `tid` of a team: its rows (y, and y + 1 for Y = 2), x-pair h, column
+// half (heights zbase + 1 ..) and addressing; false when it owns no cells (the
+// results are then those of a lane that does, safe to read with).
+//
+// Y = 1: blocks of BLOCK lanes (odd rows, half 0), [(odd rows, half 1)],
+// (even rows, half 0), [(even rows, half 1)]; Y = 2: (row pairs, half 0),
+// [(row pairs, half 1)].
+// Colour-c cell at height z of row y sits on the left (x = 2h+1) iff
+// (y + z + c) is even; its outside x neighbour is then slot own-1, else
+// own+1.  For Y = 1 the row parity is fixed per class, so the direction is
+// uniform in a wavefront; for Y = 2 left_even describes the second row.
+template <typename T, int G, int Z, int Y>
+__device__ __forceinline__ bool sor_lane(int tid, int &y, int &h, int &zbase, SorLane &ln) {
+  using C = SorCfg<T, G, Z, Y>;
+  constexpr int BLOCK = C::BLOCK, R = C::R;
+  const int blk = tid / BLOCK, li = tid - blk * BLOCK, r = li / R, h0 = li - r * R;
+  const bool active = (blk < C::NBLOCK) && (r < Geo<G>::M / 2) && (h0 < Geo<G>::HALF);
+  const int cls = Y == 1 ? blk / Z : 0;
+  y = active ? 2 * r + 1 + cls : 1;
+  h = active ? h0 : 0;
+  zbase = active ? (blk - cls * Z) * C::MH : 0;
+  const bool left_even_g = !((y + Y - 1) & 1);
+  ln.own = y * C::P + h + 1;
+  ln.left_even = left_even_g != bool(zbase & 1);
+  ln.xo_even = ln.left_even ? ln.own - 1 : ln.own + 1;
+  ln.xo_odd = ln.left_even ? ln.own + 1 : ln.own - 1;
+  ln.zoff = zbase * C::PP;
+  ln.zh = zbase != 0;
+  return active;
+}
 
 // Z = 2: reload the other-colour neighbour across the split (owned by the
 // other half's lane, updated in the previous pass) for each of the lane's rows.
@@ -325,33 +357,6 @@ __device__ __forceinline__ void sor_pass2(T (&v)[2][2][SorCfg<T, G, Z, 2>::MH + 
 // z-1, mixes pairs and stays scalar.  Heights left over: two make a pair of
 // opposite sides (scalar x additions), one stays scalar.
 // ---------------------------------------------------------------------------
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float lo2(f32x2 v) {
-  float a, b;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-  return a;
-}
-__device__ __forceinline__ float hi2(f32x2 v) {
-  float a, b;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-  return b;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-
 template <int MH>
 struct PackPairs {
   static constexpr int QUADS = MH / 4, REM = MH % 4;
@@ -383,6 +388,7 @@ struct PackState {
     const f32x2 q = v[r][c][PK::pair_of(z)];
     return PK::is_lo(z) ? lo2(q) : hi2(q);
   }
+  // the lane's arrays: x[row][colour][0..MH+1], crho[row][colour][height-1]
   template <typename V, typename R>
   __device__ __forceinline__ void load(const V &x, const R &crho) {
 #pragma unroll
@@ -404,17 +410,17 @@ struct PackState {
   }
 };
 
-template <int G, int Z, bool PHASED, int p, bool SUM, int SIDE>
-__device__ __forceinline__ void sor_pass2_packed(PackState<SorCfg<float, G, Z, 2>::MH> &st, float *s_cube,
-                                                 const SorLane &ln, float omega_6, float neg_zero,
-                                                 double (&acc4)[4]) {
+// `update(r, k, sum)` returns pair k's new values from the neighbour sums,
+// `update_one(r, sum)` the single height's.
+template <int G, int Z, bool PHASED, int p, int SIDE, typename Update, typename UpdateOne>
+__device__ __forceinline__ void pass2_packed_cells(PackState<SorCfg<float, G, Z, 2>::MH> &st, float *s_cube,
+                                                   const SorLane &ln, Update &&update, UpdateOne &&update_one) {
   using C = SorCfg<float, G, Z, 2>;
   constexpr int N = Geo<G>::N, MH = C::MH, P = C::P, PP = C::PP;
   using PK = PackPairs<MH>;
   constexpr int q = 1 - p;
   const float *nb = s_cube + q * N * PP + ln.zoff;
   float *mine = s_cube + p * N * PP + ln.zoff;
-  const f32x2 nz = pack2(neg_zero, neg_zero), w2 = pack2(omega_6, omega_6), m6 = pack2(-6.f, -6.f);
   if constexpr (Z == 2) {
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
@@ -432,9 +438,6 @@ __device__ __forceinline__ void sor_pass2_packed(PackState<SorCfg<float, G, Z, 2
   auto y_smem = [&](int r, int z) { return nb[z * PP + ln.own + (r ? 2 * P : -P)]; };
   auto x_out = [&](int r, int z) { return nb[z * PP + ln.own + r * P + (left_of(r, z) ? -1 : 1)]; };
   auto store = [&](int r, int z, float x) { mine[z * PP + ln.own + r * P] = x; };
-  auto total = [&](int r, int z, float x) {
-    if constexpr (SUM) acc4[(z + 2 * r) & 3] += (double)absval(x);
-  };
   // the six neighbours of the pair's two cells, in the reference's order
   auto pair_sum = [&](int r, int k) -> f32x2 {
     const int a = PK::lo(k), b = PK::hi(k);
@@ -453,12 +456,6 @@ __device__ __forceinline__ void sor_pass2_packed(PackState<SorCfg<float, G, Z, 2
     const float tb = add(add(hi2(t), lb ? hi2(mate) : xb), lb ? xb : hi2(mate));
     return pack2(ta, tb);
   };
-  auto pair_update = [&](int r, int k, f32x2 sum) {
-    const f32x2 res = add2(add2(sum, fma2(m6, st.v[r][p][k], nz)), st.nc[r][p][k]);
-    st.v[r][p][k] = add2(st.v[r][p][k], fma2(w2, res, nz));
-    total(r, PK::lo(k), lo2(res));
-    total(r, PK::hi(k), hi2(res));
-  };
   if constexpr (PHASED) {
     f32x2 sum[2][PK::NP];
 #pragma unroll
@@ -468,12 +465,12 @@ __device__ __forceinline__ void sor_pass2_packed(PackState<SorCfg<float, G, Z, 2
 #pragma unroll
     for (int k = 0; k < PK::NP; ++k)
 #pragma unroll
-      for (int r = 0; r < 2; ++r) pair_update(r, k, sum[r][k]);
+      for (int r = 0; r < 2; ++r) st.v[r][p][k] = update(r, k, sum[r][k]);
   } else {
 #pragma unroll
     for (int k = 0; k < PK::NP; ++k)
 #pragma unroll
-      for (int r = 0; r < 2; ++r) pair_update(r, k, pair_sum(r, k));
+      for (int r = 0; r < 2; ++r) st.v[r][p][k] = update(r, k, pair_sum(r, k));
   }
   if constexpr (PK::NS) {
     constexpr int z = PK::SINGLE;
@@ -483,9 +480,7 @@ __device__ __forceinline__ void sor_pass2_packed(PackState<SorCfg<float, G, Z, 2
       const bool left = left_of(r, z);
       float t = add(add(z_sum(r, z), r == 0 ? yreg : ysm), r == 0 ? ysm : yreg);
       t = add(add(t, left ? mate : xo), left ? xo : mate);
-      const float res = add(sub(t, mul(6.f, st.s[r][p])), st.ncs[r][p]);
-      st.s[r][p] = add(st.s[r][p], mul(omega_6, res));
-      total(r, z, res);
+      st.s[r][p] = update_one(r, t);
     }
   }
 #pragma unroll
@@ -493,6 +488,30 @@ __device__ __forceinline__ void sor_pass2_packed(PackState<SorCfg<float, G, Z, 2
     store(0, z, st.at(0, p, z));
     store(1, z, st.at(1, p, z));
   }
+}
+
+template <int G, int Z, bool PHASED, int p, bool SUM, int SIDE>
+__device__ __forceinline__ void sor_pass2_packed(PackState<SorCfg<float, G, Z, 2>::MH> &st, float *s_cube,
+                                                 const SorLane &ln, float omega_6, float neg_zero,
+                                                 double (&acc4)[4]) {
+  using PK = PackPairs<SorCfg<float, G, Z, 2>::MH>;
+  const f32x2 nz = pack2(neg_zero, neg_zero), w2 = pack2(omega_6, omega_6), m6 = pack2(-6.f, -6.f);
+  auto total = [&](int r, int z, float x) {
+    if constexpr (SUM) acc4[(z + 2 * r) & 3] += (double)absval(x);
+  };
+  pass2_packed_cells<G, Z, PHASED, p, SIDE>(
+      st, s_cube, ln,
+      [&](int r, int k, f32x2 sum) {
+        const f32x2 res = add2(add2(sum, fma2(m6, st.v[r][p][k], nz)), st.nc[r][p][k]);
+        total(r, PK::lo(k), lo2(res));
+        total(r, PK::hi(k), hi2(res));
+        return add2(st.v[r][p][k], fma2(w2, res, nz));
+      },
+      [&](int r, float sum) {
+        const float res = add(sub(sum, mul(6.f, st.s[r][p])), st.ncs[r][p]);
+        total(r, PK::SINGLE, res);
+        return add(st.s[r][p], mul(omega_6, res));
+      });
 }
 
 template <typename T, int G, int Z, int Y, bool PHASED, int p, bool SUM>
@@ -550,43 +569,25 @@ __device__ __forceinline__ void sor_solve_patch_with(const SolveArgs<T> &a, int6
   using g = Geo<G>;
   using C = SorCfg<T, G, Z, Y>;
   using S = SorSmem<T, G, Z, Y>;
-  constexpr int N = g::N, M = g::M, HALF = g::HALF, TEAM = C::TEAM, NWARP = C::NWARP;
-  constexpr int P = C::P, PP = C::PP, R = C::R, MH = C::MH, BLOCK = C::BLOCK;
+  constexpr int N = g::N, M = g::M, TEAM = C::TEAM, NWARP = C::NWARP;
+  constexpr int P = C::P, PP = C::PP, MH = C::MH;
   const int lane = tid & 31, warp = tid >> 5;
   T *s_cube = reinterpret_cast<T *>(tb);
   double *s_part = reinterpret_cast<double *>(tb + S::round(S::cube_bytes));
 
   // ---- interpolate the coarse potential into the cube (reads via L1) -----
-  interpolate<T, G, TEAM, !STAGED>(STAGED ? staged : a.pot_in + P_ * g::PN3, tid, a.int_scheme,
+  interpolate<T, G, TEAM, !STAGED>(STAGED ? staged : a.pot_in + P_ * g::PN3, tid, a.int_scheme, a.neg_zero,
                                    [s_cube](int x, int y, int z, T v) { s_cube[C::addr(x, y, z)] = v; });
   team_sync<TEAM>(team);
 
-  // ---- lane -> (rows, half, h) --------------------------------------------
-  // Y = 1: blocks of BLOCK lanes (odd rows, half 0), [(odd rows, half 1)],
-  // (even rows, half 0), [(even rows, half 1)]; Y = 2: (row pairs, half 0),
-  // [(row pairs, half 1)]
-  const int blk = tid / BLOCK, li = tid - blk * BLOCK, r = li / R, h0 = li - r * R;
-  const bool active = (blk < C::NBLOCK) && (r < M / 2) && (h0 < HALF);
-  const int cls = Y == 1 ? blk / Z : 0;
-  const int y = active ? 2 * r + 1 + cls : 1, h = active ? h0 : 0;
-  const int zbase = active ? (blk - cls * Z) * MH : 0;
-  // colour-c cell at height z of row y sits on the left (x = 2h+1) iff
-  // (y + z + c) is even; its outside x neighbour is then slot own-1, else
-  // own+1.  For Y = 1 the row parity is fixed per class, so the direction is
-  // uniform in a wavefront; for Y = 2 left_even describes the second row.
-  const bool left_even_g = !((y + Y - 1) & 1);
+  int y, h, zbase;
   SorLane ln;
-  ln.own = y * P + h + 1;
-  ln.left_even = left_even_g != bool(zbase & 1);
-  ln.xo_even = ln.left_even ? ln.own - 1 : ln.own + 1;
-  ln.xo_odd = ln.left_even ? ln.own + 1 : ln.own - 1;
-  ln.zoff = zbase * PP;
-  ln.zh = zbase != 0;
+  const bool active = sor_lane<T, G, Z, Y>(tid, y, h, zbase, ln);
 
   T v[Y][2][MH + 2];
   T crho[Y][2][MH];
-  double cr_sum = 0.0;
-  {
+  double cr_sum = 0.0;  // tolerance scale
+  if constexpr (sizeof(T) == 8) {
     const T *rho = STAGED ? staged + g::PN3 : a.rho + P_ * g::RHO3;
     const T *guess = a.guess ? a.guess + P_ * g::RHO3 : nullptr;
 #pragma unroll
@@ -614,6 +615,63 @@ __device__ __forceinline__ void sor_solve_patch_with(const SolveArgs<T> &a, int6
           if (a.init_mode != 0) v[rr][c][zz] = (a.init_mode == 2 && active) ? __ldg(guess + idx) : T(0);
         }
       }
+    }
+  } else {
+    // FP32: the two cells of a pair sit side by side, one load where the pointer
+    // allows it, and the scale is summed only where a stopping rule reads it (4096
+    // patches, gravity: ghost 4 168 -> 156 us, ghost 5 200 -> 195; the FP64 kernels
+    // came out up to 10 % slower this way)
+    const T *rho = STAGED ? staged + g::PN3 : a.rho + P_ * g::RHO3;
+    const bool pairs = (reinterpret_cast<uintptr_t>(rho) & 7) == 0;
+#pragma unroll
+    for (int rr = 0; rr < Y; ++rr) {
+      const int yr = y + rr;
+#pragma unroll
+      for (int zz = 1; zz <= MH; ++zz) {
+        const int z = zbase + zz;
+        const T *q = rho + ((z - 1) * M + (yr - 1)) * M + 2 * h;
+        float2 rv = make_float2(0.f, 0.f);
+        if (active) {
+          if (pairs) {
+            if constexpr (STAGED) rv = *reinterpret_cast<const float2 *>(q);
+            else rv = __ldg(reinterpret_cast<const float2 *>(q));
+          } else {
+            rv.x = q[0];
+            rv.y = q[1];
+          }
+        }
+        const bool left0 = ((yr + z) & 1) == 0;  // colour 0 is the left cell
+        crho[rr][0][zz - 1] = active ? mul(a.sor_const, left0 ? rv.x : rv.y) : T(0);
+        crho[rr][1][zz - 1] = active ? mul(a.sor_const, left0 ? rv.y : rv.x) : T(0);
+      }
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int zz = 0; zz < MH + 2; ++zz) v[rr][c][zz] = s_cube[(c * N + zbase + zz) * PP + ln.own + rr * P];
+    }
+    // tolerance scale: sum |Const rho| (mode 1) or sum |interpolated phi| over the
+    // updated cells, before a start mode replaces it (3)
+    if (a.stop_mode == 1 || a.stop_mode == 3) {
+#pragma unroll
+      for (int rr = 0; rr < Y; ++rr)
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+          for (int zz = 1; zz <= MH; ++zz)
+            cr_sum += (double)absval(a.stop_mode == 3 ? (active ? v[rr][c][zz] : T(0)) : crho[rr][c][zz - 1]);
+    }
+    if (a.init_mode != 0) {
+      const T *guess = a.guess ? a.guess + P_ * g::RHO3 : nullptr;
+#pragma unroll
+      for (int rr = 0; rr < Y; ++rr)
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+          for (int zz = 1; zz <= MH; ++zz) {
+            const int yr = y + rr, z = zbase + zz, x = ((yr + z + c) & 1) == 0 ? 2 * h + 1 : 2 * h + 2;
+            const int idx = ((z - 1) * M + (yr - 1)) * M + (x - 1);
+            v[rr][c][zz] = (a.init_mode == 2 && active) ? __ldg(guess + idx) : T(0);
+          }
     }
   }
   if (a.init_mode != 0 && active) {
@@ -717,28 +775,8 @@ __device__ __forceinline__ void sor_solve_patch_with(const SolveArgs<T> &a, int6
     if (a.resid) a.resid[P_] = last;
   }
 
-  // ---- output window (CPU_PoissonSolver_SOR.cpp:305-311) ------------------
-  // (edge GN a compile-time constant per GRA_GHOST_SIZE: the index split is
-  // then multiply-shift, not division)
-  auto window = [&](auto gg) {
-    constexpr int GG = decltype(gg)::value, GN = 8 + 2 * GG, shift = G - GG, GN3 = GN * GN * GN;
-    T *dst = a.pot_out + P_ * GN3;
-    for (int t = tid; t < GN3; t += TEAM) {
-      const int i = t % GN, j = (t / GN) % GN, k = t / (GN * GN);
-      dst[t] = s_cube[C::addr(i + shift, j + shift, k + shift)];
-    }
-  };
-  if (a.gra_ghost == 0)
-    window(std::integral_constant<int, 0>{});
-  else if (a.gra_ghost == 1)
-    window(std::integral_constant<int, 1>{});
-  else
-    window(std::integral_constant<int, 2>{});
-  // ---- fused gravity update (CPU_GravitySolver.cpp:34-79) -----------------
-  if (a.gra_acc) {
-    gravity_patch<T, TEAM>(a.flu + P_ * 5 * 512, tid, a.gra_const, a.p5,
-                           [s_cube](int i, int j, int k) { return s_cube[C::addr(i + G, j + G, k + G)]; });
-  }
+  // ---- output window and fused gravity update ------------------------------
+  patch_output<T, G, TEAM>(a, P_, tid, [s_cube](int x, int y, int z) { return s_cube[C::addr(x, y, z)]; });
 }
 
 template <typename T, int G, bool PHASED, int Z = 1, int Y = 1>

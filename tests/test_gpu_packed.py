@@ -48,3 +48,27 @@ def test_packed_kernels_return_the_scalar_bits(g, npatch):
         assert torch.equal(nan, nan0) and torch.equal(it, it0), v
         assert torch.equal(bits[~nan], bits0[~nan0]), v  # a NaN's payload is not specified
         assert torch.equal(torch.nan_to_num(rs, nan=-1.0), torch.nan_to_num(rs0, nan=-1.0)), v
+
+
+@pytest.mark.parametrize("rs,g,gg", [(4, 1, 1), (4, 2, 2), (4, 3, 1), (4, 4, 2), (4, 5, 1), (8, 1, 1), (8, 4, 2)])
+@pytest.mark.parametrize("scheme", [1, 2])
+def test_wide_loads_fall_back_off_their_alignment(rs, g, gg, scheme):
+    """Density pairs, coarse-potential pairs and 16-byte fluid runs: arrays one
+    element off the allocation's alignment give the aligned arrays' bits."""
+    torch = pytest.importorskip("torch")
+    from gpg.lib import solve_device
+    dev = torch.device("cuda:0")
+    d = make_patches(37, g, seed=60 + g, gra_ghost=gg, dtype=np.float32 if rs == 4 else np.float64)
+    p = default_params(rs, g, scheme, gra_ghost=gg, p5_gradient=int(gg == 2))
+
+    def off(t, k):
+        buf = torch.empty(t.numel() + k, dtype=t.dtype, device=dev)
+        buf[k:] = t.reshape(-1)
+        return buf[k:].view(t.shape)
+
+    t = {k: torch.from_numpy(d[k]).to(dev) for k in ("rho", "pot_in", "flu")}
+    want = solve_device(p, t["rho"], t["pot_in"], flu=t["flu"].clone())
+    for k in (1, 2, 3):
+        got = solve_device(p, off(t["rho"], k), off(t["pot_in"], k), flu=off(t["flu"], k))
+        for a, b in zip(got, want):
+            assert torch.equal(a, b), k
