@@ -50,18 +50,6 @@ int fail(int status, const char *fmt, ...) {
 // ---------------------------------------------------------------------------
 // launch configuration per (precision, ghost size)
 // ---------------------------------------------------------------------------
-// MG threads per CTA (one patch per CTA), from a B200 sweep of 128-1024
-// threads per (precision, ghost size); results do not depend on it.  FP32:
-// ghost 3 with 5-point gravity, 16384 patches: 128 threads 0.918 ms, 256 0.957,
-// 512 1.065; ghost 5: 512 threads 0.522 ms, 256 0.542, 128 0.606; ghost 4: 256.
-// FP64 (about 160 registers per thread): ghost 3, 2048 patches: 128 threads
-// 1.228 ms, 256 1.366; ghost 4 and 5: 256 (512 and 1024 spill); ghost 1-2: 128.
-template <typename T, int G>
-constexpr int mg_threads() {
-  if constexpr (sizeof(T) == 4) return G <= 3 ? 128 : (G == 4 ? 256 : 512);
-  return G <= 3 ? 128 : 256;
-}
-
 // Kernel attributes, set once per (kernel instantiation, device) -- they
 // belong to a device's context -- by the first call on that device (the
 // caller owns the state): the dynamic shared memory size and the max-shared
@@ -378,12 +366,12 @@ int prepare_solve_kernels(const gpg_params &q) {
 
 template <typename T, int G>
 int launch_mg(const gpg::SolveArgs<T> &a, cudaStream_t s) {
-  constexpr int NT = mg_threads<T, G>();
-  const size_t smem = gpg::MgSmem<T, G, NT>::bytes;
-  auto fn = gpg::mg_kernel<T, G, NT>;
+  using K = gpg::MgCfg<T, G>;
+  const size_t smem = K::bytes;
+  auto fn = gpg::mg_kernel<T, G>;
   static AttrOnce attr;
   if (int rc = ensure_smem(fn, smem, attr)) return rc;
-  fn<<<(unsigned)a.npatch, NT, smem, s>>>(a);
+  fn<<<(unsigned)a.npatch, K::TEAM, smem, s>>>(a);
   GPG_CUDA(cudaGetLastError());
   return GPG_OK;
 }
