@@ -87,12 +87,34 @@ def check(rc: int):
         raise GpgError(rc, msg.decode() if msg else "")
 
 
-def _tptr(t):
+def tensor_ptr(t):
+    """Address of a contiguous CUDA tensor (None stays None), as ctypes takes it."""
     if t is None:
         return None
     if not t.is_cuda or not t.is_contiguous():
         raise ValueError("device API needs contiguous CUDA tensors")
-    return C.c_void_p(t.data_ptr())
+    return t.data_ptr()
+
+
+def stream_ptr(stream, device_index: int) -> int:
+    """Handle of `stream` (a torch.cuda.Stream), or of the device's current
+    stream when None.  The raw handle is read without building a Stream object:
+    a small solve's launch is otherwise shorter than the call around it (256
+    patches at ghost 1: 12 us of kernel, 12.8 us of Python before, 5 now)."""
+    if stream is not None:
+        return stream.cuda_stream
+    return torch_module()._C._cuda_getCurrentRawStream(device_index)
+
+
+_torch = None
+
+
+def torch_module():
+    global _torch
+    if _torch is None:
+        import torch
+        _torch = torch
+    return _torch
 
 
 def solve_device(p: GpgParams, rho=None, pot_in=None, pot_out=None, flu=None, guess=None, iters=None,
@@ -101,26 +123,23 @@ def solve_device(p: GpgParams, rho=None, pot_in=None, pot_out=None, flu=None, gu
 
     Allocates pot_out / iters / resid when not given (iters and resid always
     returned).  `stream` is a torch.cuda.Stream or None (current stream)."""
-    import torch
+    torch = torch_module()
     dt = torch.float32 if p.real_size == 4 else torch.float64
     src = rho if rho is not None else pot_out
     n = src.shape[0] if npatch is None else npatch
     dev = src.device
-    gn = 8 + 2 * p.gra_ghost
     if pot_out is None:
+        gn = 8 + 2 * p.gra_ghost
         pot_out = torch.empty((n, gn, gn, gn), dtype=dt, device=dev)
     if iters is None:
         iters = torch.empty(n, dtype=torch.int32, device=dev)
     if resid is None:
         resid = torch.empty(n, dtype=torch.float64, device=dev)
     for t in (rho, pot_in, pot_out, flu, guess):
-        if t is not None and t.dtype != dt:
+        if t is not None and t.dtype is not dt:
             raise TypeError(f"expected {dt}, got {t.dtype}")
-    s = stream if stream is not None else torch.cuda.current_stream(dev)
-    rc = library().gpg_poisson_gravity_device(
-        C.byref(p), int(n), _tptr(rho), _tptr(pot_in), _tptr(pot_out), _tptr(flu), _tptr(guess),
-        _tptr(iters), _tptr(resid), C.c_void_p(s.cuda_stream))
-    check(rc)
+    ptrs = [tensor_ptr(t) for t in (rho, pot_in, pot_out, flu, guess, iters, resid)]
+    check(library().gpg_poisson_gravity_device(C.byref(p), int(n), *ptrs, stream_ptr(stream, dev.index)))
     return pot_out, flu, iters, resid
 
 
@@ -221,7 +240,7 @@ def make_batch_groups(p: GpgParams, groups: list[dict]):
         for k, f in (("rho", "d_rho"), ("pot_in", "d_pot_in"), ("pot_out", "d_pot_out"), ("flu", "d_flu"),
                      ("guess", "d_guess"), ("iters", "d_iters"), ("resid", "d_resid")):
             t = g.get(k)
-            setattr(a, f, None if t is None else _tptr(t).value)
+            setattr(a, f, tensor_ptr(t))
         a.sor_omega = g.get("omega", 0.0)
     return arr
 
@@ -229,11 +248,9 @@ def make_batch_groups(p: GpgParams, groups: list[dict]):
 def solve_batch_device(p: GpgParams, groups: list[dict], counter, stream=None):
     """One persistent launch over groups of different ghost sizes.  `counter`:
     a 1-element int32 CUDA tensor used as the work-queue counter."""
-    import torch
     arr = make_batch_groups(p, groups)
-    s = stream if stream is not None else torch.cuda.current_stream(counter.device)
-    check(library().gpg_solve_batch_device(C.byref(p), len(groups), arr, _tptr(counter),
-                                           C.c_void_p(s.cuda_stream)))
+    check(library().gpg_solve_batch_device(C.byref(p), len(groups), arr, tensor_ptr(counter),
+                                           stream_ptr(stream, counter.device.index)))
 
 
 PLAN_PERSISTENT, PLAN_CONCURRENT = 0, 1
@@ -252,9 +269,7 @@ class BatchPlan:
                                               mode))
 
     def launch(self, stream=None):
-        import torch
-        s = stream if stream is not None else torch.cuda.current_stream()
-        check(library().gpg_batch_plan_launch(self._plan, C.c_void_p(s.cuda_stream)))
+        check(library().gpg_batch_plan_launch(self._plan, stream_ptr(stream, torch_module().cuda.current_device())))
 
     def close(self):
         if self._plan:

@@ -12,14 +12,18 @@ import ctypes as C
 import numpy as np
 
 from .abi import GpgParams
-from .lib import GpgError, library
+from .lib import GpgError, library, stream_ptr, torch_module
 
 NPARAMS = 4 * 64 * 64
 
 
+_lib = None
+
+
 def _lin_lib():
-    lib = library()
-    if not getattr(lib, "_lin_sigs", False):
+    global _lib
+    if _lib is None:
+        lib = library()
         vp = C.c_void_p
         P = C.POINTER(GpgParams)
         sig = {
@@ -43,8 +47,8 @@ def _lin_lib():
             f = getattr(lib, name)
             f.restype = res
             f.argtypes = args
-        lib._lin_sigs = True
-    return lib
+        _lib = lib
+    return _lib
 
 
 def _check(rc):
@@ -58,7 +62,7 @@ def _p(t):
         return None
     if not t.is_cuda or not t.is_contiguous():
         raise ValueError("the learned correction needs contiguous CUDA tensors")
-    return C.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 class LinearGuess:
@@ -74,8 +78,7 @@ class LinearGuess:
 
     @staticmethod
     def _s(stream):
-        import torch
-        return C.c_void_p((stream or torch.cuda.current_stream()).cuda_stream)
+        return stream_ptr(stream, torch_module().cuda.current_device())
 
     def params(self) -> np.ndarray:
         out = np.empty(self.nparams, dtype=np.float32)

@@ -5,14 +5,18 @@ import ctypes as C
 
 import numpy as np
 
-from .lib import GpgError, library
+from .lib import GpgError, library, stream_ptr, torch_module
 
 LAYERS = ((8, 32), (32, 32), (32, 32), (32, 16))   # (cin, cout), padded
 
 
+_lib = None
+
+
 def _net_lib():
-    lib = library()
-    if not getattr(lib, "_net_sigs", False):
+    global _lib
+    if _lib is None:
+        lib = library()
         vp = C.c_void_p
         sig = {
             "gpg_net_create": (C.c_int, [C.POINTER(vp), C.c_int, C.c_uint64, C.c_int]),
@@ -33,8 +37,8 @@ def _net_lib():
             f = getattr(lib, name)
             f.restype = res
             f.argtypes = args
-        lib._net_sigs = True
-    return lib
+        _lib = lib
+    return _lib
 
 
 def _check(rc):
@@ -81,8 +85,7 @@ class Net:
 
     @staticmethod
     def _s(stream):
-        import torch
-        return C.c_void_p((stream or torch.cuda.current_stream()).cuda_stream)
+        return stream_ptr(stream, torch_module().cuda.current_device())
 
     def predict(self, rho, pot_in, guess, cnst: float, stream=None, fused: bool = True):
         """Interior guess; `fused` False runs the per-layer kernels instead."""
