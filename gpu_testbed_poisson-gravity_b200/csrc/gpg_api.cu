@@ -192,8 +192,7 @@ int launch_sor_v(const gpg::SolveArgs<T> &a, cudaStream_t s) {
       return fail(GPG_ERR_UNSUPPORTED, "SOR variant needs %d threads per CTA (registers allow %d)", threads,
                   max_threads);
     const int64_t grid = (a.npatch + PPC - 1) / PPC;
-    fn<<<(unsigned)grid, threads, smem, s>>>(a);
-    GPG_CUDA(cudaGetLastError());
+    GPG_CUDA(gpg::launch_after(fn, (unsigned)grid, threads, smem, s, a));
     return GPG_OK;
   }
 }
@@ -244,8 +243,7 @@ int launch_staged_v(const gpg::SolveArgs<T> &a, cudaStream_t s) {
     }
     const int64_t need = (a.npatch + TPC - 1) / TPC;
     const int64_t grid = std::min<int64_t>(need, resident[dev]);
-    fn<<<(unsigned)grid, TPC * TEAM, SS::bytes, s>>>(a);
-    GPG_CUDA(cudaGetLastError());
+    GPG_CUDA(gpg::launch_after(fn, (unsigned)grid, TPC * TEAM, SS::bytes, s, a));
     return GPG_OK;
   }
 }
@@ -371,8 +369,7 @@ int launch_mg(const gpg::SolveArgs<T> &a, cudaStream_t s) {
   auto fn = gpg::mg_kernel<T, G>;
   static AttrOnce attr;
   if (int rc = ensure_smem(fn, smem, attr)) return rc;
-  fn<<<(unsigned)a.npatch, K::TEAM, smem, s>>>(a);
-  GPG_CUDA(cudaGetLastError());
+  GPG_CUDA(gpg::launch_after(fn, (unsigned)a.npatch, K::TEAM, smem, s, a));
   return GPG_OK;
 }
 

@@ -78,6 +78,7 @@ __global__ void lin_pack_kernel(const float *__restrict__ w, __nv_bfloat16 *__re
 
 // one Adam step and the operand tiles of the new weights
 __global__ void lin_adam_kernel(const gpg::AdamArgs a, __nv_bfloat16 *__restrict__ tiles) {
+  gpg::pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < kParams) tiles[tile_index(i)] = __float2bfloat16_rn(gpg::adam_update(a, i));
 }
@@ -118,6 +119,7 @@ __global__ void __launch_bounds__(kGradThreads) lin_grad_kernel(const float *__r
   extern __shared__ __align__(16) unsigned char lin_smem[];
   GradSmem &sm = *reinterpret_cast<GradSmem *>(lin_smem);
   const int b = blockIdx.x, tid = threadIdx.x, c = class_of(b);
+  gpg::pdl_wait();
   for (int i = tid; i < kK * kK; i += kGradThreads) sm.wt[i % kK][i / kK] = w[c * kK * kK + i];
   const int r0 = (tid & 15) * 4;             // 4 rows of E and of G
   const int p0 = (tid >> 4) * 4;             // 4 patches of E
@@ -191,6 +193,7 @@ __global__ void __launch_bounds__(kGradThreads) lin_grad_kernel(const float *__r
         for (int j = 0; j < 4; ++j) g[i][j] = fmaf(xe[i], yu[j], g[i][j]);
     }
   }
+  gpg::pdl_trigger();
   const int slot = blockIdx.y * 8 + b;
 #pragma unroll
   for (int i = 0; i < 4; ++i)
@@ -215,6 +218,8 @@ __global__ void __launch_bounds__(256) lin_reduce_kernel(const float *__restrict
   __shared__ float sums[4][64];
   const int v = threadIdx.x & 63, q = threadIdx.x >> 6, i = blockIdx.x * 64 + v;
   const int c = i / (kK * kK), rk = i % (kK * kK);
+  gpg::pdl_wait();
+  gpg::pdl_trigger();
   float s = 0.f;
 #pragma unroll
   for (int b = 0; b < 8; ++b) {
@@ -458,10 +463,10 @@ extern "C" int gpg_lin_gradients(gpg_lin *l, int npatch, const float *d_u, const
   LIN_CUDA(cudaSetDevice(l->device));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int nsplit = std::min(kGradSplit, (npatch + kChunk - 1) / kChunk);
-  lin_grad_kernel<<<dim3(8, nsplit), kGradThreads, sizeof(GradSmem), s>>>(d_u, d_t, l->params, npatch, l->part, l->loss_part);
-  lin_reduce_kernel<<<kParams / 64, 256, 0, s>>>(l->part, l->loss_part, nsplit, npatch, d_grad ? d_grad : l->grad,
-                                                  d_loss ? d_loss : l->loss);
-  LIN_CUDA(cudaGetLastError());
+  LIN_CUDA(gpg::launch_after(lin_grad_kernel, dim3(8, nsplit), kGradThreads, sizeof(GradSmem), s, d_u, d_t, l->params,
+                             npatch, l->part, l->loss_part));
+  LIN_CUDA(gpg::launch_after(lin_reduce_kernel, kParams / 64, 256, 0, s, l->part, l->loss_part, nsplit, npatch,
+                             d_grad ? d_grad : l->grad, d_loss ? d_loss : l->loss));
   return GPG_OK;
 }
 
@@ -470,9 +475,8 @@ int lin_adam(gpg_lin *l, const float *grad, float lr, cudaStream_t s) {
   l->step += 1;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - std::pow(b1, float(l->step)), c2 = 1.f - std::pow(b2, float(l->step));
-  lin_adam_kernel<<<kParams / 256, 256, 0, s>>>(
-      gpg::AdamArgs{l->params, l->adam_m, l->adam_v, grad, lr, b1, b2, 1e-8f, c1, c2}, l->tiles);
-  LIN_CUDA(cudaGetLastError());
+  LIN_CUDA(gpg::launch_after(lin_adam_kernel, kParams / 256, 256, 0, s,
+                             gpg::AdamArgs{l->params, l->adam_m, l->adam_v, grad, lr, b1, b2, 1e-8f, c1, c2}, l->tiles));
   return GPG_OK;
 }
 }  // namespace

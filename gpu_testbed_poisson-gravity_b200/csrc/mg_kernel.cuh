@@ -406,6 +406,7 @@ __global__ void __launch_bounds__(MgCfg<T, G>::TEAM, (MgCfg<T, G>::blocks)) mg_k
   double *s_red = reinterpret_cast<double *>(smem_raw + K::red);
   const int tid = threadIdx.x;
   const int64_t P_ = blockIdx.x;
+  pdl_wait();
   prefetch_patch<T, G, NT>(a, P_, tid);
 
   // level-0 solution = interpolated cube; coarse boundaries 0; prolongation weights
@@ -619,6 +620,7 @@ __global__ void __launch_bounds__(MgCfg<T, G>::TEAM, (MgCfg<T, G>::blocks)) mg_k
     if (a.iters) a.iters[P_] = iter;
     if (a.resid) a.resid[P_] = err;
   }
+  pdl_trigger();
   patch_output<T, G, NT>(a, P_, tid, [s_cube](int x, int y, int z) { return s_cube[C::addr(x, y, z)]; });
 }
 
