@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "../../include/gpg.h"
+#include "args.cuh"
 #include "common.cuh"
 #include "convnet_kernels.cuh"
 #include "convnet_infer.cuh"
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(256) input_kernel(const float *__restrict__ rh
   __shared__ float cube[kCells];
   __shared__ float red[8];
   const int64_t p = blockIdx.x;
+  gpg::pdl_wait();
   gpg::interpolate<float, 1, 256>(pot_in + p * gpg::Geo<1>::PN3, threadIdx.x, 4, neg_zero,
                                   [](int x, int y, int z, float v) { cube[(z * 10 + y) * 10 + x] = v; });
   __syncthreads();
@@ -97,6 +99,7 @@ __global__ void __launch_bounds__(256) input_kernel(const float *__restrict__ rh
   float s = red[0];
   for (int w = 1; w < 8; ++w) s = fmaxf(s, red[w]);
   if (!(s > 0.f)) s = 1.f;
+  gpg::pdl_trigger();
   if (threadIdx.x == 0) scale[p] = s;
   for (int v = threadIdx.x; v < kCells; v += 256) {
     const int x = v % 10, y = (v / 10) % 10, z = v / 100;
@@ -131,6 +134,8 @@ __global__ void __launch_bounds__(256) reduce_kernel(const ReduceArgs a) {
   const int v = threadIdx.x & 63, q = threadIdx.x >> 6;
   constexpr int kOut4 = 16;  // output channels of layer 4, padded
   const int i = blockIdx.x * 64 + v, total = a.first[kLayers];
+  gpg::pdl_wait();
+  gpg::pdl_trigger();
   float s = 0.f;
   if (i < total) {
     int l = 0;
@@ -251,8 +256,7 @@ int launch_conv1(ConvArgs a, cudaStream_t s) {
   using C = gpg::net::Conv1Cfg;
   if (int rc = set_attr_once(gpg::net::conv1_kernel, C::bytes, once)) return rc;
   a.zc = unit_planes(a.npatch, kEdge, kEdge);
-  gpg::net::conv1_kernel<<<(unsigned)unit_grid(a.npatch, kEdge, a.zc), C::THREADS, C::bytes, s>>>(a);
-  NET_CUDA(cudaGetLastError());
+  NET_CUDA(gpg::launch_after(gpg::net::conv1_kernel, (unsigned)unit_grid(a.npatch, kEdge, a.zc), C::THREADS, C::bytes, s, a));
   return GPG_OK;
 }
 
@@ -266,8 +270,7 @@ int launch_conv(ConvArgs a, cudaStream_t s, int *grid_out = nullptr) {
   a.zc = unit_planes(a.npatch, nz, nz);
   const int grid = unit_grid(a.npatch, nz, a.zc);
   if (grid_out) *grid_out = grid;
-  fn<<<(unsigned)grid, C::THREADS, C::bytes, s>>>(a);
-  NET_CUDA(cudaGetLastError());
+  NET_CUDA(gpg::launch_after(fn, (unsigned)grid, C::THREADS, C::bytes, s, a));
   return GPG_OK;
 }
 
@@ -280,8 +283,7 @@ int launch_wgrad(WgradArgs a, cudaStream_t s, int *grid_out) {
   a.zc = unit_planes(a.npatch, kEdge, W::ZMAX);
   const int grid = unit_grid(a.npatch, kEdge, a.zc);
   *grid_out = grid;
-  fn<<<(unsigned)grid, W::THREADS, W::bytes, s>>>(a);
-  NET_CUDA(cudaGetLastError());
+  NET_CUDA(gpg::launch_after(fn, (unsigned)grid, W::THREADS, W::bytes, s, a));
   return GPG_OK;
 }
 
@@ -327,9 +329,11 @@ ConvArgs conv_args(gpg_net *n, int64_t npatch) {
 }
 
 // input planes and the activations of layers 1-3
+// (the training kernels launch ahead of the end of the one before: barrier and
+// TMEM set-up overlap its tail; a training step of 1024 patches 615 -> 590 us, of
+// 333 308 -> 263, of 32 147 -> 110)
 int forward_hidden(gpg_net *n, int64_t npatch, const float *rho, const float *pot_in, float cnst, cudaStream_t s) {
-  input_kernel<<<(unsigned)npatch, 256, 0, s>>>(rho, pot_in, n->x0, n->scale, cnst, -0.f);
-  NET_CUDA(cudaGetLastError());
+  NET_CUDA(gpg::launch_after(input_kernel, (unsigned)npatch, 256, 0, s, rho, pot_in, n->x0, n->scale, cnst, -0.f));
   ConvArgs a = conv_args(n, npatch);
   for (int l = 0; l < 3; ++l) {
     a.x = l == 0 ? n->x0 : n->act[l - 1];
@@ -386,8 +390,7 @@ int gradients(gpg_net *n, int64_t npatch, const float *rho, const float *pot_in,
                         : launch_conv<32, 32, gpg::net::EPI_MASK>(a, s, &r.nb[l - 1]))
       return rc;
   }
-  reduce_kernel<<<(unsigned)((kParams + 63) / 64), 256, 0, s>>>(r);
-  NET_CUDA(cudaGetLastError());
+  NET_CUDA(gpg::launch_after(reduce_kernel, (unsigned)((kParams + 63) / 64), 256, 0, s, r));
   return GPG_OK;
 }
 

@@ -35,6 +35,7 @@
 
 #include <cstdint>
 
+#include "common.cuh"
 #include "tc_common.cuh"
 
 namespace gpg {
@@ -283,6 +284,7 @@ __global__ void __launch_bounds__(Conv1Cfg::THREADS) conv1_kernel(const ConvArgs
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = *s_tmem;
+  pdl_wait();
   const int zc = a.zc, upp = kEdge / zc;
   const int64_t nunit = a.npatch * upp;
 
@@ -439,6 +441,7 @@ __global__ void __launch_bounds__(ConvCfg<CIN, NOUT>::THREADS) conv_kernel(const
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
+  pdl_wait();
   const int zc = a.zc, upp = E::NZ / zc;
   const int64_t nunit = a.npatch * upp, first = blockIdx.x + int64_t(stream) * gridDim.x,
                 step = int64_t(STREAMS) * gridDim.x;
@@ -545,6 +548,7 @@ __global__ void __launch_bounds__(ConvCfg<CIN, NOUT>::THREADS) conv_kernel(const
       q0 += uint32_t(w1 - w0 + 1);
     }
     if (!ok) *s_abort = 1;
+    pdl_trigger();
     epi.finish(reinterpret_cast<float *>(smem + C::red_off), warp, lane);
   }
   tc::fence_before_sync();
@@ -650,6 +654,7 @@ __global__ void __launch_bounds__(WgradCfg<CIN, LAST>::THREADS) wgrad_kernel(con
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = *s_tmem;
+  pdl_wait();
   const int zc = a.zc, upp = kEdge / zc;
   const int64_t nunit = a.npatch * upp;
   const bool any = blockIdx.x < nunit;
@@ -714,6 +719,7 @@ __global__ void __launch_bounds__(WgradCfg<CIN, LAST>::THREADS) wgrad_kernel(con
     if (!wait.ok) *s_abort = 1;
     tc::mma_commit_warp(done);
   }
+  pdl_trigger();
   // every accumulation has ended (bounded wait, one thread)
   if (tid == 160) tc::mbar_wait(done, 0, a.err);
   __syncwarp();
