@@ -29,12 +29,16 @@
 // one is solved.  Per batch, every team interpolates its patch from the
 // staged copy into its shared cube, forms r0 for its cells, folds it and
 // writes the 8 block vectors (BF16) into its half's MMA operand tile; one
-// thread per half issues 16 tcgen05.mma (M 128 = two class matrices stacked,
+// warp per half issues 16 tcgen05.mma (M 128 = two class matrices stacked,
 // N 16 = the 8 patches of two blocks side by side, K 64) against the weight
 // tiles, which stay in shared memory for the whole kernel; the teams read the
 // FP32 results back from TMEM, unfold their own patch, add the correction to
 // the cube and run the ordinary sweeps, stopping rule, output window and
-// (optionally) gravity update of sor_solve_patch_with.
+// (optionally) gravity update of sor_solve_patch_with.  Bound by the latency of a
+// batch's chain (interpolation, fold, MMAs, unfold, about one sweep) with 4 warps a
+// scheduler: 61 % of the issue slots; packing the transforms' instructions changed
+// nothing.  The MMAs are issued by the whole of a half's first warp (one lane alone
+// takes 81 cycles an MMA for them, not 43; 306 -> 303 us).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -54,11 +58,9 @@ constexpr int kTileBytes = 128 * kK * 2;       // one A tile (BF16): 16 KB
 // of padding put consecutive chunks on different banks for the operand stores)
 constexpr int kChunkB = kN * 16 + 16;
 constexpr int kGroupBytes = (kK / 8) * kChunkB;
-// team scratch: interior cell (z, y, x) at z * kScrPZ + y * 8 + x (plane pitch
-// padded from 64 so that lane-cell and mirror-orbit accesses spread over the
-// banks), block results at b * 64 + o
-constexpr int kScrPZ = 66;
-constexpr int kScrWords = 8 * kScrPZ;
+// team scratch: interior cell (z, y, x) at word scr_cell(), result o of block b at
+// word scr_block(); a bijection each
+constexpr int kScrWords = 512;
 constexpr int kHalfCols = kGroups * kN;        // TMEM columns of one group of teams: 64
 constexpr int kParams = 4 * kK * kK;           // 16,384
 constexpr int kFeatureGain = 17;               // log2 of the training features' extra scale
@@ -81,8 +83,18 @@ __host__ __device__ constexpr int perm_orbit(int o, int t) {
   const int k = o >> 4, j = (o >> 2) & 3, i = o & 3;
   return t == 0 ? o : (t == 1 ? (k << 4) | (i << 2) | j : (t == 2 ? (i << 4) | (j << 2) | k : (j << 4) | (k << 2) | i));
 }
-// scratch word of interior cell (z, y, x)
-__host__ __device__ constexpr int scr_cell(int z, int y, int x) { return z * kScrPZ + y * 8 + x; }
+// scratch word of interior cell (z, y, x).  The banks are those of y and x; of a
+// warp's accesses, the ones by orbit (z in a pair, y and x in a half) leave x bit 2
+// and the ones by lane cell (z in {z0, z0 + 4}, y and x of one parity) leave y bit 0
+// and x bit 0 unused, so z bit 0, y bit 2 and z bit 2 are folded into those: 32
+// different banks in both (a padded plane pitch had two to a bank in either; 65536
+// patches 308 -> 294 us)
+__host__ __device__ constexpr int scr_cell(int z, int y, int x) {
+  return z * 64 + (y ^ (y >> 2)) * 8 + (x ^ ((z & 1) << 2) ^ (z >> 2));
+}
+// scratch word of result o of block b: the writes run along an axis-permuted orbit
+// index, whose bit 5 would otherwise fall out of the banks
+__host__ __device__ constexpr int scr_block(int b, int o) { return b * 64 + (o ^ ((o >> 5) * 10)); }
 // scratch word of orbit o's image under mirror s = (sz, sy, sx)
 __host__ __device__ constexpr int orbit_cell(int o, int s) {
   const int k = o >> 4, j = (o >> 2) & 3, i = o & 3;
@@ -211,9 +223,10 @@ __device__ __forceinline__ void lane_xyz(const SorLaneState<float, 1, 2, 2> &st,
 }
 // its scratch word
 __device__ __forceinline__ int lane_cell(const SorLaneState<float, 1, 2, 2> &st, int r, int p, int z) {
-  int cz, cy, cx;
-  lane_xyz(st, r, p, z, cz, cy, cx);
-  return scr_cell(cz, cy, cx);
+  // the lane's part; row, side and height change bits of their own
+  const int base = st.zbase * 64 + ((st.y - 1) ^ ((st.y - 1) >> 2)) * 8 + ((2 * st.h) ^ (st.zbase >> 2));
+  const int side = (1 + r + z + p) & 1;  // y starts odd, zbase is even
+  return (base ^ (r * 8 + (side ^ (((z - 1) & 1) << 2)))) + (z - 1) * 64;
 }
 
 template <bool FEATURES, int HALVES, bool STAGE>
@@ -237,10 +250,6 @@ __global__ void __launch_bounds__(Shape<HALVES, STAGE>::kThreads, 1) lin_sor_ker
 
   uint32_t tmem = 0;
   if constexpr (!FEATURES) {
-    // weight tiles: resident for the whole kernel
-    const uint4 *src = reinterpret_cast<const uint4 *>(a.wtiles);
-    uint4 *dst = reinterpret_cast<uint4 *>(sA);
-    for (int i = tid; i < 2 * kTileBytes / 16; i += kThreads) dst[i] = src[i];
     if (tid == 0) {
       for (int i = 0; i < Layout::kBars; ++i) tc::mbar_init(&bars[i], 1);
       tc::mbar_fence_init();
@@ -249,6 +258,11 @@ __global__ void __launch_bounds__(Shape<HALVES, STAGE>::kThreads, 1) lin_sor_ker
       tc::tmem_alloc(s_tmem, kTmemCols);
       tc::tmem_relinquish();
     }
+    pdl_wait();
+    // weight tiles: resident for the whole kernel
+    const uint4 *src = reinterpret_cast<const uint4 *>(a.wtiles);
+    uint4 *dst = reinterpret_cast<uint4 *>(sA);
+    for (int i = tid; i < 2 * kTileBytes / 16; i += kThreads) dst[i] = src[i];
     tc::fence_proxy_async_smem();
     tc::fence_before_sync();
     __syncthreads();
@@ -388,7 +402,7 @@ __global__ void __launch_bounds__(Shape<HALVES, STAGE>::kThreads, 1) lin_sor_ker
           }
         tc::fence_proxy_async_smem();
         half_bar(half);  // operands complete; the previous batch's results were read
-        if (wl == 0 && lane == 0) {
+        if (wl == 0) {
           tc::fence_after_sync();
           const uint32_t a0 = tc::smem_u32(sA), b0 = tc::smem_u32(sB);
 #pragma unroll
@@ -397,9 +411,9 @@ __global__ void __launch_bounds__(Shape<HALVES, STAGE>::kThreads, 1) lin_sor_ker
             for (int ks = 0; ks < kK / 16; ++ks) {
               const uint64_t ad = tc::smem_desc(a0 + (g ? kTileBytes : 0) + 2 * ks * 2048, 2048, 128);
               const uint64_t bd = tc::smem_desc(b0 + g * kGroupBytes + 2 * ks * kChunkB, kChunkB, 128);
-              tc::mma_bf16(tmem + uint32_t(g * kN), ad, bd, kIdesc, ks > 0 ? 1u : 0u);
+              tc::mma_bf16_warp(tmem + uint32_t(g * kN), ad, bd, kIdesc, ks > 0 ? 1u : 0u);
             }
-          tc::mma_commit(bar_mma);
+          tc::mma_commit_warp(bar_mma);
         }
         if (!tc::mbar_wait(bar_mma, phase, a.err)) late = true;
         last_parity = phase;
@@ -416,7 +430,7 @@ __global__ void __launch_bounds__(Shape<HALVES, STAGE>::kThreads, 1) lin_sor_ker
             tmem_ld8(tmem + (uint32_t(32 * q) << 16) + uint32_t(g * kN + side * kHalfWarps), val);
             tc::tmem_wait_ld();
             const int b = block_of(g, side), o = perm_orbit(row, perm_of(b));
-            float *dst = s_scr + size_t(half) * kHalfWarps * kScrWords + b * 64 + o;
+            float *dst = s_scr + size_t(half) * kHalfWarps * kScrWords + scr_block(b, o);
 #pragma unroll
             for (int n = 0; n < kHalfWarps; ++n) dst[n * kScrWords] = val[n];
           }
@@ -429,7 +443,7 @@ __global__ void __launch_bounds__(Shape<HALVES, STAGE>::kThreads, 1) lin_sor_ker
         for (int oo = 0; oo < 2; ++oo) {
           const int o = lane + 32 * oo;
 #pragma unroll
-          for (int b = 0; b < 8; ++b) d[oo][b] = scr[b * 64 + o];
+          for (int b = 0; b < 8; ++b) d[oo][b] = scr[scr_block(b, o)];
           hadamard8(d[oo]);
         }
         __syncwarp();
@@ -462,6 +476,7 @@ __global__ void __launch_bounds__(Shape<HALVES, STAGE>::kThreads, 1) lin_sor_ker
       sor_solve_patch_with<float, 1, false, 2, 2, false, false>(a.s, P_, 0, lane, tb, real, hook);
     }
   }
+  pdl_trigger();
   if constexpr (!FEATURES) {
     // after a timed-out wait the MMAs may still run: wait for the half's last
     // commit (bounded) before the accumulator columns are released

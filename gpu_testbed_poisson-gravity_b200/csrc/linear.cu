@@ -417,16 +417,17 @@ extern "C" int gpg_lin_solve_device(gpg_lin *l, const gpg_params *p, int npatch,
   a.err = l->err;
   a.probe_polls = l->probe_polls;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  // the set-up overlaps the end of the kernel before (300 patches, back to back:
+  // 16.7 -> 13.6 us; 4096 28.7 -> 25.4)
   if (l->variant == 0) {
     using SH = gpg::lin::Shape<2, true>;
-    gpg::lin::lin_sor_kernel<false, 2, true><<<lin_grid(2, l->grid[0], npatch), SH::kThreads,
-                                               gpg::lin::Layout<2, true>::bytes, s>>>(a);
+    LIN_CUDA(gpg::launch_after(gpg::lin::lin_sor_kernel<false, 2, true>, lin_grid(2, l->grid[0], npatch), SH::kThreads,
+                               gpg::lin::Layout<2, true>::bytes, s, a));
   } else {
     using SH = gpg::lin::Shape<3, false>;
-    gpg::lin::lin_sor_kernel<false, 3, false><<<lin_grid(3, l->grid[1], npatch), SH::kThreads,
-                                                gpg::lin::Layout<3, false>::bytes, s>>>(a);
+    LIN_CUDA(gpg::launch_after(gpg::lin::lin_sor_kernel<false, 3, false>, lin_grid(3, l->grid[1], npatch), SH::kThreads,
+                               gpg::lin::Layout<3, false>::bytes, s, a));
   }
-  LIN_CUDA(cudaGetLastError());
   return GPG_OK;
 }
 

@@ -620,7 +620,8 @@ __device__ __forceinline__ void sor_solve_patch_with(const SolveArgs<T> &a, int6
     // FP32: the two cells of a pair sit side by side, one load where the pointer
     // allows it, and the scale is summed only where a stopping rule reads it (4096
     // patches, gravity: ghost 4 168 -> 156 us, ghost 5 200 -> 195; the FP64 kernels
-    // came out up to 10 % slower this way)
+    // came out up to 10 % slower this way).  Staged inputs stay scalar: the learned
+    // start's kernel was slower with pairs (65536 patches 294 us, 299 with)
     const T *rho = STAGED ? staged + g::PN3 : a.rho + P_ * g::RHO3;
     const bool pairs = (reinterpret_cast<uintptr_t>(rho) & 7) == 0;
 #pragma unroll
@@ -632,9 +633,8 @@ __device__ __forceinline__ void sor_solve_patch_with(const SolveArgs<T> &a, int6
         const T *q = rho + ((z - 1) * M + (yr - 1)) * M + 2 * h;
         float2 rv = make_float2(0.f, 0.f);
         if (active) {
-          if (pairs) {
-            if constexpr (STAGED) rv = *reinterpret_cast<const float2 *>(q);
-            else rv = __ldg(reinterpret_cast<const float2 *>(q));
+          if (!STAGED && pairs) {
+            rv = __ldg(reinterpret_cast<const float2 *>(q));
           } else {
             rv.x = q[0];
             rv.y = q[1];

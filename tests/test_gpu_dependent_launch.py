@@ -68,3 +68,33 @@ def test_chained_solves(rs, npatch, g):
     torch.cuda.synchronize()
     for a, b in zip(again, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("npatch", [1, 9, 300, 5000])
+@pytest.mark.parametrize("variant", [0, 1])
+def test_chained_learned_solves(npatch, variant):
+    torch = pytest.importorskip("torch")
+    from gpg.linear import LinearGuess
+    dev = torch.device("cuda:0")
+    d = make_patches(npatch, 1, seed=3, dtype=np.float32)
+    rho, pin = (torch.from_numpy(d[k]).to(dev) for k in ("rho", "pot_in"))
+    lin = LinearGuess(max_batch=64)
+    lin.set_params(0.01 * np.random.default_rng(5).standard_normal(lin.nparams).astype(np.float32))
+    lin.set_variant(variant)
+    p = default_params(4, 1, GPG_SOR, gra_ghost=0, gra_acc=0, sor_max_iter=6)
+
+    def chain(wait):
+        out, src = [], rho  # each solve's density is the potential before it
+        for _ in range(4):
+            out.append(lin.solve(p, src, pin))
+            src = out[-1][0]
+            if wait:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return out
+
+    for a, b in zip(chain(True), chain(False)):
+        for k in (0, 2, 3):
+            assert torch.equal(a[k], b[k])
+    lin.check()
+    lin.close()
