@@ -94,8 +94,8 @@ __global__ void lin_adam_kernel(const gpg::AdamArgs a, __nv_bfloat16 *__restrict
 // features are loaded while the current one is multiplied.  grid.y = 37 puts
 // two CTAs on each of 148 SMs (8 x 37 = 296) and bounds the partial sums to 4.8
 // MB, which the second kernel adds in a fixed order.
-// Training step (gradient, Adam, operand tiles) of 2048 patches: 1212 -> 24.6
-// us, of which the host's calls are about 22 (64 patches take the same).
+// Training step (gradient, Adam, operand tiles) of 2048 patches: 1212 -> 18.6
+// us (24.6 without the launches' overlap, see launch_after).
 // (A thread that walks all patches for its row and column, as before, waits
 // for 6144 dependent steps.)
 // The error e = W u - t sums k in order, as the single-row form did.

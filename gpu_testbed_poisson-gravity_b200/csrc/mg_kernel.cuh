@@ -307,9 +307,9 @@ __device__ __forceinline__ void mg_coarse(const SolveArgs<T> &a, T *sol, T *rhs,
     pairs.defect(s, def, dh);
     team_sync<NT>(0);
     mg_restrict<T, NT, n, nn>(
-        [def](int bz, int by, int bx) {
+        [def](int bz, int by, int bx) GPG_INLINE {
           const T *f = def + (bz * n + by) * n + bx;
-          return [f](int tz, int ty, int tx) { return f[(tz * n + ty) * n + tx]; };
+          return [f](int tz, int ty, int tx) GPG_INLINE { return f[(tz * n + ty) * n + tx]; };
         },
         rn, tid);
     if constexpr (lv + 1 < LV::L - 1)
@@ -366,7 +366,7 @@ __device__ __forceinline__ void pass2_cells(T (&v)[2][2][SorCfg<T, G, Z, 2>::MH 
   // sum of the six neighbours of row r's colour-p cell at height z; yreg is
   // the y neighbour held in registers (y0+1 for row 0, y1-1 for row 1), ysm
   // the one read from shared memory
-  auto nbsum = [&](int z, int r, T yreg, T ysm, bool left, T xo) -> T {
+  auto nbsum = [&](int z, int r, T yreg, T ysm, bool left, T xo) GPG_INLINE -> T {
     const T mate = v[r][1 - p][z];
     const T yp = r == 0 ? yreg : ysm, ym = r == 0 ? ysm : yreg;
     const T xp = left ? mate : xo, xm = left ? xo : mate;
@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(MgCfg<T, G>::TEAM, (MgCfg<T, G>::blocks)) mg_k
 
   // level-0 solution = interpolated cube; coarse boundaries 0; prolongation weights
   interpolate<T, G, NT>(a.pot_in + P_ * g::PN3, tid, a.int_scheme, a.neg_zero,
-                        [s_cube](int x, int y, int z, T v) { s_cube[C::addr(x, y, z)] = v; });
+                        [s_cube](int x, int y, int z, T v) GPG_INLINE { s_cube[C::addr(x, y, z)] = v; });
   for (int t = tid; t < LV::coarse; t += NT) s_sol[t] = T(0);
   for (int f = tid + 1; f <= M; f += NT) mg_weights(f, divide(T(n1 - 1), T(N - 1)), s_w0[f], s_w1[f], s_base[f]);
   team_sync<NT>(0);
@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(MgCfg<T, G>::TEAM, (MgCfg<T, G>::blocks)) mg_k
   // whether its colour-c cell of row r at local height zz is the left one of the
   // pair (y is odd; the column half matters only where it is an odd number of heights)
   const int odd_base = (MH & 1) ? zbase & 1 : 0;
-  auto is_left = [&](int r, int c, int zz) { return ((1 + r + odd_base + zz + c) & 1) == 0; };
+  auto is_left = [&](int r, int c, int zz) GPG_INLINE { return ((1 + r + odd_base + zz + c) & 1) == 0; };
   // the lane's columns and Poi_Coeff * rho, [row][colour][height]
   T v[2][2][MH + 2], rhs[2][2][MH];
 #pragma unroll
@@ -440,9 +440,9 @@ __global__ void __launch_bounds__(MgCfg<T, G>::TEAM, (MgCfg<T, G>::blocks)) mg_k
   const T dh = a.dh, dh2 = mul(dh, dh), m_dh2 = divide(T(-1), dh2), one_six = divide(T(1), T(6));
 
   // red-black sweeps of level 0
-  auto smooth = [&](int sweeps) {
+  auto smooth = [&](int sweeps) GPG_INLINE {
     if (sweeps <= 0) return;
-    auto by_side = [&](auto f) {  // the side of the lane's cells, where that is warp-uniform
+    auto by_side = [&](auto f) GPG_INLINE {  // the side of the lane's cells, where that is warp-uniform
       if constexpr (C::HALF_UNIFORM) {
         if (ln.left_even) f(std::integral_constant<int, 1>{});
         else f(std::integral_constant<int, 0>{});
@@ -456,16 +456,16 @@ __global__ void __launch_bounds__(MgCfg<T, G>::TEAM, (MgCfg<T, G>::blocks)) mg_k
       const f32x2 nz = pack2(a.neg_zero, a.neg_zero), d2 = pack2(dh2, dh2), s6 = pack2(one_six, one_six);
 #pragma unroll 1
       for (int q = 0; q < sweeps; ++q) {
-        auto pass = [&](auto pc) {
+        auto pass = [&](auto pc) GPG_INLINE {
           constexpr int p = decltype(pc)::value;
           if (active)
-            by_side([&](auto side) {
+            by_side([&](auto side) GPG_INLINE {
               pass2_packed_cells<G, Z, false, p, decltype(side)::value>(
                   st, s_cube, ln,
-                  [&](int r, int k, f32x2 sum) {
+                  [&](int r, int k, f32x2 sum) GPG_INLINE {
                     return fma2(s6, add2(sum, fma2(d2, st.nc[r][p][k], nz)), nz);
                   },
-                  [&](int r, float sum) { return mul(one_six, add(sum, mul(dh2, st.ncs[r][p]))); });
+                  [&](int r, float sum) GPG_INLINE { return mul(one_six, add(sum, mul(dh2, st.ncs[r][p]))); });
             });
           team_sync<NT>(0);
         };
@@ -481,11 +481,11 @@ __global__ void __launch_bounds__(MgCfg<T, G>::TEAM, (MgCfg<T, G>::blocks)) mg_k
     } else {
 #pragma unroll 1
       for (int q = 0; q < sweeps; ++q) {
-        auto pass = [&](auto pc) {
+        auto pass = [&](auto pc) GPG_INLINE {
           constexpr int p = decltype(pc)::value;
           if (active)
-            by_side([&](auto side) {
-              pass2_cells<T, G, Z, p, decltype(side)::value>(v, s_cube, ln, [&](int r, int z, T sum) {
+            by_side([&](auto side) GPG_INLINE {
+              pass2_cells<T, G, Z, p, decltype(side)::value>(v, s_cube, ln, [&](int r, int z, T sum) GPG_INLINE {
                 return mul(one_six, sub(sum, mul(dh2, rhs[r][p][z - 1])));
               });
             });
@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(MgCfg<T, G>::TEAM, (MgCfg<T, G>::blocks)) mg_k
     }
   };
   // f(r, zz, defect) for the lane's colour-c cells (the other colour's cube planes hold the solution)
-  auto defects = [&](auto cc, auto f) {
+  auto defects = [&](auto cc, auto f) GPG_INLINE {
     constexpr int c = decltype(cc)::value;
     const T *nb0 = s_cube + (1 - c) * N * PP + ln.zoff, *nb = nb0 + ln.own;
     sor_reload_split<T, MH, PP, P, 2, c>(v, nb0, ln);
@@ -515,7 +515,9 @@ __global__ void __launch_bounds__(MgCfg<T, G>::TEAM, (MgCfg<T, G>::blocks)) mg_k
   };
   constexpr std::integral_constant<int, 0> c0{};
   constexpr std::integral_constant<int, 1> c1{};
-  auto place = [&](int r, int c, int zz) -> T & { return s_cube[(c * N + zbase + zz) * PP + ln.own + r * P]; };
+  auto place = [&](int r, int c, int zz) GPG_INLINE -> T & {
+    return s_cube[(c * N + zbase + zz) * PP + ln.own + r * P];
+  };
 
   int iter = 0;
   double err = (double)FLT_MAX;
@@ -527,9 +529,9 @@ __global__ void __launch_bounds__(MgCfg<T, G>::TEAM, (MgCfg<T, G>::blocks)) mg_k
       // alone: colour 1 (from colour 0's planes) waits in registers until colour 0's
       // planes are free for colour 0's own
       T d[2][MH];
-      if (active) defects(c1, [&](int r, int zz, T x) { d[r][zz - 1] = x; });
+      if (active) defects(c1, [&](int r, int zz, T x) GPG_INLINE { d[r][zz - 1] = x; });
       team_sync<NT>(0);
-      if (active) defects(c0, [&](int r, int zz, T x) { place(r, 0, zz) = x; });
+      if (active) defects(c0, [&](int r, int zz, T x) GPG_INLINE { place(r, 0, zz) = x; });
       team_sync<NT>(0);
       if (active) {
 #pragma unroll
@@ -540,12 +542,12 @@ __global__ void __launch_bounds__(MgCfg<T, G>::TEAM, (MgCfg<T, G>::blocks)) mg_k
       team_sync<NT>(0);
     }
     mg_restrict<T, NT, N, n1>(
-        [s_cube](int bz, int by, int bx) {
+        [s_cube](int bz, int by, int bx) GPG_INLINE {
           // cells with an even step count share a colour; the middle x sits in the next slot iff bx is even
           const int s = (bx + by + bz + 1) & 1, step = !(bx & 1);
           const T *even = s_cube + (s * N + bz) * PP + by * P + ((bx + 1) >> 1);
           const T *odd = even + (s ? -N * PP : N * PP);
-          return [even, odd, step](int tz, int ty, int tx) {
+          return [even, odd, step](int tz, int ty, int tx) GPG_INLINE {
             const T *q = ((tz + ty + tx) & 1) ? odd : even;
             return q[tz * PP + ty * P + (tx == 0 ? 0 : tx == 2 ? 1 : step)];
           };
@@ -603,11 +605,11 @@ __global__ void __launch_bounds__(MgCfg<T, G>::TEAM, (MgCfg<T, G>::blocks)) mg_k
     smooth(a.mg_npost);
     double sd = 0, ss = 0;
     if (active) {
-      defects(c0, [&](int r, int zz, T x) {
+      defects(c0, [&](int r, int zz, T x) GPG_INLINE {
         sd += (double)absval(x);
         ss += (double)absval(v[r][0][zz]);
       });
-      defects(c1, [&](int r, int zz, T x) {
+      defects(c1, [&](int r, int zz, T x) GPG_INLINE {
         sd += (double)absval(x);
         ss += (double)absval(v[r][1][zz]);
       });
@@ -621,7 +623,7 @@ __global__ void __launch_bounds__(MgCfg<T, G>::TEAM, (MgCfg<T, G>::blocks)) mg_k
     if (a.resid) a.resid[P_] = err;
   }
   pdl_trigger();
-  patch_output<T, G, NT>(a, P_, tid, [s_cube](int x, int y, int z) { return s_cube[C::addr(x, y, z)]; });
+  patch_output<T, G, NT>(a, P_, tid, [s_cube](int x, int y, int z) GPG_INLINE { return s_cube[C::addr(x, y, z)]; });
 }
 
 }  // namespace gpg

@@ -281,7 +281,7 @@ __device__ __forceinline__ void sor_pass2(T (&v)[2][2][SorCfg<T, G, Z, 2>::MH + 
   // sum of the six neighbours of row r's colour-p cell at height z; yreg is
   // the y neighbour held in registers (y0+1 for row 0, y1-1 for row 1), ysm
   // the one read from shared memory
-  auto nbsum = [&](int z, int r, T yreg, T ysm, bool left, T xo) -> T {
+  auto nbsum = [&](int z, int r, T yreg, T ysm, bool left, T xo) GPG_INLINE -> T {
     const T mate = v[r][1 - p][z];
     const T yp = r == 0 ? yreg : ysm, ym = r == 0 ? ysm : yreg;
     const T xp = left ? mate : xo, xm = left ? xo : mate;
@@ -433,13 +433,13 @@ __device__ __forceinline__ void pass2_packed_cells(PackState<SorCfg<float, G, Z,
   }
   constexpr bool RT = (Z == 2) && (MH & 1);
   const bool le = SIDE >= 0 ? SIDE == 1 : (RT ? ln.left_even : true);
-  auto left_of = [&](int r, int z) { return ((((z + p) & 1) == 0) == le) == (r == 1); };
-  auto z_sum = [&](int r, int z) { return add(st.at(r, q, z + 1), st.at(r, q, z - 1)); };
-  auto y_smem = [&](int r, int z) { return nb[z * PP + ln.own + (r ? 2 * P : -P)]; };
-  auto x_out = [&](int r, int z) { return nb[z * PP + ln.own + r * P + (left_of(r, z) ? -1 : 1)]; };
-  auto store = [&](int r, int z, float x) { mine[z * PP + ln.own + r * P] = x; };
+  auto left_of = [&](int r, int z) GPG_INLINE { return ((((z + p) & 1) == 0) == le) == (r == 1); };
+  auto z_sum = [&](int r, int z) GPG_INLINE { return add(st.at(r, q, z + 1), st.at(r, q, z - 1)); };
+  auto y_smem = [&](int r, int z) GPG_INLINE { return nb[z * PP + ln.own + (r ? 2 * P : -P)]; };
+  auto x_out = [&](int r, int z) GPG_INLINE { return nb[z * PP + ln.own + r * P + (left_of(r, z) ? -1 : 1)]; };
+  auto store = [&](int r, int z, float x) GPG_INLINE { mine[z * PP + ln.own + r * P] = x; };
   // the six neighbours of the pair's two cells, in the reference's order
-  auto pair_sum = [&](int r, int k) -> f32x2 {
+  auto pair_sum = [&](int r, int k) GPG_INLINE -> f32x2 {
     const int a = PK::lo(k), b = PK::hi(k);
     f32x2 t = pack2(z_sum(r, a), z_sum(r, b));
     const f32x2 yreg = st.v[1 - r][q][k], ysm = pack2(y_smem(r, a), y_smem(r, b));
@@ -496,18 +496,18 @@ __device__ __forceinline__ void sor_pass2_packed(PackState<SorCfg<float, G, Z, 2
                                                  double (&acc4)[4]) {
   using PK = PackPairs<SorCfg<float, G, Z, 2>::MH>;
   const f32x2 nz = pack2(neg_zero, neg_zero), w2 = pack2(omega_6, omega_6), m6 = pack2(-6.f, -6.f);
-  auto total = [&](int r, int z, float x) {
+  auto total = [&](int r, int z, float x) GPG_INLINE {
     if constexpr (SUM) acc4[(z + 2 * r) & 3] += (double)absval(x);
   };
   pass2_packed_cells<G, Z, PHASED, p, SIDE>(
       st, s_cube, ln,
-      [&](int r, int k, f32x2 sum) {
+      [&](int r, int k, f32x2 sum) GPG_INLINE {
         const f32x2 res = add2(add2(sum, fma2(m6, st.v[r][p][k], nz)), st.nc[r][p][k]);
         total(r, PK::lo(k), lo2(res));
         total(r, PK::hi(k), hi2(res));
         return add2(st.v[r][p][k], fma2(w2, res, nz));
       },
-      [&](int r, float sum) {
+      [&](int r, float sum) GPG_INLINE {
         const float res = add(sub(sum, mul(6.f, st.s[r][p])), st.ncs[r][p]);
         total(r, PK::SINGLE, res);
         return add(st.s[r][p], mul(omega_6, res));
@@ -577,7 +577,7 @@ __device__ __forceinline__ void sor_solve_patch_with(const SolveArgs<T> &a, int6
 
   // ---- interpolate the coarse potential into the cube (reads via L1) -----
   interpolate<T, G, TEAM, !STAGED>(STAGED ? staged : a.pot_in + P_ * g::PN3, tid, a.int_scheme, a.neg_zero,
-                                   [s_cube](int x, int y, int z, T v) { s_cube[C::addr(x, y, z)] = v; });
+                                   [s_cube](int x, int y, int z, T v) GPG_INLINE { s_cube[C::addr(x, y, z)] = v; });
   team_sync<TEAM>(team);
 
   int y, h, zbase;
@@ -718,7 +718,7 @@ __device__ __forceinline__ void sor_solve_patch_with(const SolveArgs<T> &a, int6
     // combined in a fixed order, so the total is deterministic and identical
     // for a patch solved alone or in a batch
     double acc4[4] = {0.0, 0.0, 0.0, 0.0};
-    auto pass = [&](auto colour_c, auto sum_c) {
+    auto pass = [&](auto colour_c, auto sum_c) GPG_INLINE {
       constexpr int p = decltype(colour_c)::value;
       constexpr bool SUM = decltype(sum_c)::value;
       if (!active) return;
@@ -777,7 +777,7 @@ __device__ __forceinline__ void sor_solve_patch_with(const SolveArgs<T> &a, int6
 
   if (trigger) pdl_trigger();
   // ---- output window and fused gravity update ------------------------------
-  patch_output<T, G, TEAM>(a, P_, tid, [s_cube](int x, int y, int z) { return s_cube[C::addr(x, y, z)]; });
+  patch_output<T, G, TEAM>(a, P_, tid, [s_cube](int x, int y, int z) GPG_INLINE { return s_cube[C::addr(x, y, z)]; });
 }
 
 template <typename T, int G, bool PHASED, int Z = 1, int Y = 1>
@@ -844,7 +844,7 @@ __global__ void __launch_bounds__(TPC *SorCfg<T, G, Z, Y>::TEAM, (StagedSmem<T, 
     tc::mbar_fence_init();
   }
   __syncthreads();
-  auto stage = [&](int64_t P) {  // one thread: patch P's inputs -> stg
+  auto stage = [&](int64_t P) GPG_INLINE {  // one thread: patch P's inputs -> stg
     tc::mbar_arrive_expect_tx(bar, uint32_t(sizeof(T) * SS::stage_elems));
     tc::bulk_load(stg, a.pot_in + P * g::PN3, uint32_t(sizeof(T) * g::PN3), bar);
     tc::bulk_load(stg + g::PN3, a.rho + P * g::RHO3, uint32_t(sizeof(T) * g::RHO3), bar);
@@ -860,7 +860,7 @@ __global__ void __launch_bounds__(TPC *SorCfg<T, G, Z, Y>::TEAM, (StagedSmem<T, 
     const int64_t next = P_ + stride;
     sor_solve_patch_with<T, G, PHASED, Z, Y, true>(
         a, P_, team, tid, tb, true,
-        [&](const auto &) {
+        [&](const auto &) GPG_INLINE {
           // the staged inputs are in the cube and registers: fetch the next patch
           if (tid == 0 && next < a.npatch) {
             tc::fence_proxy_async_smem();
