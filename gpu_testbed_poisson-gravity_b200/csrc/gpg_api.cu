@@ -124,8 +124,10 @@ std::atomic<bool> g_sor_pinned[2][6] = {};
 // up to max_npatch patches: FP32 ghost 1 at 256 patches 16.5 -> 12.4 us per
 // launch, ghost 2 16.0 -> 12.5, ghost 3 18.6 -> 16.6; FP32 ghost 5 runs the
 // large-launch layout at every size, ghost 4 the split column up to 1024 (45.6
-// us; the whole one 45.8, at 256 patches 20.6 and 22.7).  FP64 ghost 2 at 256
-// 53.6 -> 39.1, ghost 4 at 64 72.7 -> 59.6.  FP64 ghost 5 keeps the
+// us; the whole one 45.8, at 256 patches 20.6 and 22.7) and, with one patch per SM,
+// one row per lane (64 patches 14.5 -> 12.1, 100 16.5 -> 14.0; 200 18.6 -> 18.9).
+// FP64 ghost 2 at 256 53.6 -> 39.1, ghost 4 the staged kernel while half the SMs
+// have a patch (64: 65.7 -> 60.3; 150: 79.0 -> 81.0).  FP64 ghost 5 keeps the
 // unstaged v11 up to 1024 patches: the staged kernel hands patches out at a
 // fixed stride, and 1024 patches over its 296 teams leave some teams a fourth
 // patch (333 vs 360 us; through the CUAPI path, 4 streams of 1024 patches,
@@ -133,10 +135,10 @@ std::atomic<bool> g_sor_pinned[2][6] = {};
 struct SorSmall {
   int max_npatch, variant;
 };
-constexpr SorSmall kSorSmall[2][6] = {
-    // ghost:  -       1          2          3         4          5
-    {{0, 0}, {2048, 7}, {512, 6}, {512, 7}, {1024, 11}, {0, 0}},     // float
-    {{0, 0}, {256, 8}, {256, 7}, {0, 0}, {256, 14}, {1024, 11}},     // double
+constexpr SorSmall kSorSmall[2][6][2] = {
+    // ghost 0 (none), 1, 2, 3, 4, 5; the smaller limit first, 0 none
+    {{}, {{2048, 7}}, {{512, 6}}, {{512, 7}}, {{148, 6}, {1024, 11}}, {}},  // float
+    {{}, {{256, 8}}, {{256, 7}}, {}, {{74, 15}}, {{1024, 11}}},             // double
 };
 std::once_flag g_tune_once;
 
@@ -277,8 +279,13 @@ struct SharedSms {
 // the variant a launch of npatch patches runs
 inline int sor_variant_for(bool f64, int g, int64_t npatch) {
   int v = g_sor_variant[f64][g].load(std::memory_order_relaxed);
-  const SorSmall &sm = kSorSmall[f64][g];
-  if (!g_sor_pinned[f64][g].load(std::memory_order_relaxed) && npatch <= sm.max_npatch) v = sm.variant;
+  if (!g_sor_pinned[f64][g].load(std::memory_order_relaxed)) {
+    for (const SorSmall &sm : kSorSmall[f64][g])
+      if (npatch <= sm.max_npatch) {
+        v = sm.variant;
+        break;
+      }
+  }
   if (t_shared_sms && kSorVariantStaged[v]) v = v == 14 ? 10 : (v == 15 ? 11 : 13);  // same layout, unstaged
   return v;
 }
@@ -340,9 +347,11 @@ template <typename T, int G>
 int prepare_sor() {
   std::call_once(g_tune_once, load_tune_file);
   constexpr bool f64 = sizeof(T) == 8;
-  const int large = sor_variant_for(f64, G, std::numeric_limits<int64_t>::max()), small = sor_variant_for(f64, G, 0);
-  if (int rc = prepare_sor_variant<T, G>(large)) return rc;
-  return small == large ? GPG_OK : prepare_sor_variant<T, G>(small);
+  if (int rc = prepare_sor_variant<T, G>(sor_variant_for(f64, G, std::numeric_limits<int64_t>::max()))) return rc;
+  for (const SorSmall &sm : kSorSmall[f64][G])
+    if (sm.max_npatch > 0)
+      if (int rc = prepare_sor_variant<T, G>(sor_variant_for(f64, G, sm.max_npatch))) return rc;
+  return GPG_OK;
 }
 
 template <typename T>
@@ -362,15 +371,37 @@ int prepare_solve_kernels(const gpg_params &q) {
   return q.real_size == 4 ? prepare_sor_typed<float>(q.ghost) : prepare_sor_typed<double>(q.ghost);
 }
 
+// Launches of up to this many patches run the wide multigrid kernel: with one or
+// two CTAs per SM the time is one patch's latency, which the helping threads
+// shorten.  us per launch, as wide as level 0 / wide: 64 patches FP32 ghost 1 17.1 /
+// 12.9, 2 14.8 / 12.8, 3 16.7 / 14.8, 5 29.2 / 21.3, FP64 ghost 1 60.0 / 53.8, 5 191 /
+// 167; 296 patches FP32 17.0 / 13.1, 15.1 / 14.8, 17.2 / 16.8, 31.4 / 26.9, FP64 ghost
+// 1 62.2 / 55.9, 5 217 / 334 (148: 193 / 169).  Elsewhere the wide form gains
+// nothing (FP32 ghost 4) or spills (FP64 ghost 3 89 / 117 at 64 patches, 4 126 / 154).
+template <typename T, int G>
+constexpr int kMgWide = sizeof(T) == 4 ? (G == 4 ? 0 : 296) : (G == 1 ? 296 : (G == 5 ? 148 : 0));
+
+template <typename T, int G, bool WIDE>
+int prepare_mg() {
+  static AttrOnce attr;
+  return ensure_smem(gpg::mg_kernel<T, G, WIDE>, gpg::MgCfg<T, G, WIDE>::bytes, attr);
+}
+
+template <typename T, int G, bool WIDE>
+int run_mg(const gpg::SolveArgs<T> &a, cudaStream_t s) {
+  using K = gpg::MgCfg<T, G, WIDE>;
+  GPG_CUDA(gpg::launch_after(gpg::mg_kernel<T, G, WIDE>, (unsigned)a.npatch, K::TEAM, K::bytes, s, a));
+  return GPG_OK;
+}
+
 template <typename T, int G>
 int launch_mg(const gpg::SolveArgs<T> &a, cudaStream_t s) {
-  using K = gpg::MgCfg<T, G>;
-  const size_t smem = K::bytes;
-  auto fn = gpg::mg_kernel<T, G>;
-  static AttrOnce attr;
-  if (int rc = ensure_smem(fn, smem, attr)) return rc;
-  GPG_CUDA(gpg::launch_after(fn, (unsigned)a.npatch, K::TEAM, smem, s, a));
-  return GPG_OK;
+  if (int rc = prepare_mg<T, G, false>()) return rc;
+  if constexpr (kMgWide<T, G> > 0) {
+    if (int rc = prepare_mg<T, G, true>()) return rc;
+    if (a.npatch <= kMgWide<T, G>) return run_mg<T, G, true>(a, s);
+  }
+  return run_mg<T, G, false>(a, s);
 }
 
 template <typename T, int GG>

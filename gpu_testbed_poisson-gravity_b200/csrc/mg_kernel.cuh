@@ -68,12 +68,14 @@ struct MgLevels {
   static_assert(L >= 3, "a level between the finest and the bottom");
 };
 
-template <typename T, int G>
+template <typename T, int G, bool WIDE = false>
 struct MgCfg {
   static constexpr int Z = 2;  // lanes per column
   using C = SorCfg<T, G, Z, 2>;
   using LV = MgLevels<G>;
-  static constexpr int TEAM = C::TEAM;
+  // threads of the CTA: the level-0 layout's, or (WIDE) at least twice as many, the
+  // others helping with all but the level-0 sweeps
+  static constexpr int TEAM = !WIDE ? C::TEAM : (2 * C::TEAM < 128 ? 128 : 2 * C::TEAM);
   static constexpr size_t round(size_t b) { return (b + 15) / 16 * 16; }
   static constexpr size_t cube = 0;                                         // level 0: solution, or its defect
   static constexpr size_t sol = cube + round(sizeof(T) * C::CUBE);          // levels 1..
@@ -390,11 +392,12 @@ __device__ __forceinline__ void pass2_cells(T (&v)[2][2][SorCfg<T, G, Z, 2>::MH 
   }
 }
 
-template <typename T, int G>
-__global__ void __launch_bounds__(MgCfg<T, G>::TEAM, (MgCfg<T, G>::blocks)) mg_kernel(const SolveArgs<T> a) {
+template <typename T, int G, bool WIDE = false>
+__global__ void __launch_bounds__(MgCfg<T, G, WIDE>::TEAM, (MgCfg<T, G, WIDE>::blocks))
+    mg_kernel(const SolveArgs<T> a) {
   using LV = MgLevels<G>;
   using g = Geo<G>;
-  using K = MgCfg<T, G>;
+  using K = MgCfg<T, G, WIDE>;
   using C = typename K::C;
   constexpr int N = g::N, M = g::M, Z = K::Z, NT = K::TEAM, P = C::P, PP = C::PP, MH = C::MH;
   constexpr int n1 = LV::size(1);

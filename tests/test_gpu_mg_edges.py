@@ -33,3 +33,31 @@ def test_mg_loops_match_the_oracle(rs, g):
         assert np.array_equal(pot.cpu().numpy(), op), kw
         assert np.array_equal(flu.cpu().numpy(), of), kw
         np.testing.assert_allclose(err.cpu().numpy(), oe, rtol=1e-12, err_msg=str(kw))
+
+
+@pytest.mark.parametrize("rs", [4, 8])
+@pytest.mark.parametrize("g", [1, 2, 3, 4, 5])
+def test_launch_sizes_agree(rs, g):
+    """Small launches run a kernel with more threads per patch: the same bits for a
+    patch solved in a launch of either kind, and the oracle's."""
+    torch = pytest.importorskip("torch")
+    from gpg.lib import solve_device
+    from oracle.oracle import run_oracle
+    dev = torch.device("cuda:0")
+    d = make_patches(297, g, seed=90 + g, dtype=np.float32 if rs == 4 else np.float64)
+    p = default_params(rs, g, GPG_MG)
+    t = {k: torch.from_numpy(d[k]).to(dev) for k in ("rho", "pot_in", "flu")}
+
+    def solve(n):
+        flu = t["flu"][:n].clone()
+        pot, _, it, err = solve_device(p, t["rho"][:n], t["pot_in"][:n], flu=flu)
+        return pot, flu, it, err
+
+    want = solve(297)
+    for n in (1, 148, 149, 296):
+        for a, b in zip(solve(n), want):
+            assert torch.equal(a, b[:n])
+    op, of, oi, _ = run_oracle(p, d["rho"][:12], d["pot_in"][:12], flu=d["flu"][:12].copy(), accum_f64=True)
+    assert np.array_equal(want[0][:12].cpu().numpy(), op)
+    assert np.array_equal(want[1][:12].cpu().numpy(), of)
+    assert np.array_equal(want[2][:12].cpu().numpy(), oi)
