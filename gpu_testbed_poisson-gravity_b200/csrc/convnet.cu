@@ -498,7 +498,10 @@ extern "C" int gpg_net_create(gpg_net **out, int max_batch, uint64_t seed, int d
     delete n;
     return nfail(GPG_ERR_CUDA, "upload: %s", cudaGetErrorString(e));
   }
-  if (int rc = repack(n, 0)) {
+  int rc = repack(n, 0);
+  if (!rc && cudaDeviceSynchronize() != cudaSuccess)
+    rc = nfail(GPG_ERR_CUDA, "set-up: %s", cudaGetErrorString(cudaGetLastError()));
+  if (rc) {
     free_net(n);
     delete n;
     return rc;
@@ -519,6 +522,7 @@ extern "C" int gpg_net_destroy(gpg_net *n) {
 extern "C" int gpg_net_get_params(gpg_net *n, float *host) {
   if (!n || !host) return nfail(GPG_ERR_INVALID, "NULL argument");
   NET_CUDA(cudaSetDevice(n->device));
+  NET_CUDA(cudaDeviceSynchronize());  // training steps on any stream
   NET_CUDA(cudaMemcpy(host, n->params, kParams * 4, cudaMemcpyDeviceToHost));
   return GPG_OK;
 }
@@ -526,11 +530,15 @@ extern "C" int gpg_net_get_params(gpg_net *n, float *host) {
 extern "C" int gpg_net_set_params(gpg_net *n, const float *host) {
   if (!n || !host) return nfail(GPG_ERR_INVALID, "NULL argument");
   NET_CUDA(cudaSetDevice(n->device));
+  // calls before and after may be on streams that the default stream does not order
+  NET_CUDA(cudaDeviceSynchronize());
   NET_CUDA(cudaMemcpy(n->params, host, kParams * 4, cudaMemcpyHostToDevice));
   NET_CUDA(cudaMemset(n->adam_m, 0, kParams * 4));
   NET_CUDA(cudaMemset(n->adam_v, 0, kParams * 4));
   n->step = 0;
-  return repack(n, 0);
+  if (int rc = repack(n, 0)) return rc;
+  NET_CUDA(cudaDeviceSynchronize());
+  return GPG_OK;
 }
 
 extern "C" int gpg_net_check(gpg_net *n) {

@@ -381,6 +381,7 @@ extern "C" int gpg_lin_destroy(gpg_lin *l) {
 extern "C" int gpg_lin_get_params(gpg_lin *l, float *host) {
   if (!l || !host) return lfail(GPG_ERR_INVALID, "NULL argument");
   LIN_CUDA(cudaSetDevice(l->device));
+  LIN_CUDA(cudaDeviceSynchronize());  // training steps on any stream
   LIN_CUDA(cudaMemcpy(host, l->params, kParams * 4, cudaMemcpyDeviceToHost));
   return GPG_OK;
 }
@@ -388,6 +389,8 @@ extern "C" int gpg_lin_get_params(gpg_lin *l, float *host) {
 extern "C" int gpg_lin_set_params(gpg_lin *l, const float *host) {
   if (!l || !host) return lfail(GPG_ERR_INVALID, "NULL argument");
   LIN_CUDA(cudaSetDevice(l->device));
+  // calls before and after may be on streams that the default stream does not order
+  LIN_CUDA(cudaDeviceSynchronize());
   LIN_CUDA(cudaMemcpy(l->params, host, kParams * 4, cudaMemcpyHostToDevice));
   LIN_CUDA(cudaMemset(l->adam_m, 0, kParams * 4));
   LIN_CUDA(cudaMemset(l->adam_v, 0, kParams * 4));
