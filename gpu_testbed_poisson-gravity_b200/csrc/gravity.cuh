@@ -44,15 +44,16 @@ __device__ __forceinline__ void gravity_cell(int i, int j, int k, T gra_const, i
 // per thread and step: 128 FP32 runs instead of 512 cells, so that a team of 96
 // threads waits for two rounds of loads and not six.  flu points at one patch
 // [5][8][8][8]; a pointer off the 16-byte alignment takes the values one by one.
-template <typename T>
+// CELLS = 1: single cells.
+template <typename T, int CELLS = 16 / sizeof(T)>
 struct FluidRun {
-  static constexpr int W = 16 / sizeof(T), RUNS = 512 / W;
+  static constexpr int W = CELLS, RUNS = 512 / W;
   T q[5][W];  // component, cell
   __device__ __forceinline__ void load(const T *flu, int run, bool aligned) {
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
       const T *src = flu + c * 512 + run * W;
-      if (aligned) {
+      if (W > 1 && aligned) {
         *reinterpret_cast<uint4 *>(q[c]) = *reinterpret_cast<const uint4 *>(src);
       } else {
 #pragma unroll
@@ -64,7 +65,7 @@ struct FluidRun {
 #pragma unroll
     for (int c = 1; c < 5; ++c) {  // the density is read only
       T *dst = flu + c * 512 + run * W;
-      if (aligned) {
+      if (W > 1 && aligned) {
         *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(q[c]);
       } else {
 #pragma unroll
@@ -90,12 +91,11 @@ __device__ __forceinline__ bool aligned16(const void *p) { return (reinterpret_c
 template <typename T, int NT, typename Phi>
 __device__ __forceinline__ void gravity_patch(T *__restrict__ flu, int tid, T gra_const, int p5,
                                               Phi phi) {
-  const bool al = aligned16(flu);
-  for (int run = tid; run < FluidRun<T>::RUNS; run += NT) {
-    FluidRun<T> f;
-    f.load(flu, run, al);
-    f.update(run, gra_const, p5, phi);
-    f.store(flu, run, al);
+  for (int cell = tid; cell < 512; cell += NT) {
+    FluidRun<T, 1> f;
+    f.load(flu, cell, false);
+    f.update(cell, gra_const, p5, phi);
+    f.store(flu, cell, false);
   }
 }
 
@@ -151,7 +151,10 @@ __device__ __forceinline__ void prefetch_patch(const SolveArgs<T> &a, int64_t P,
 
 // Gravity alone (Poisson off): the potential comes from pot_out
 // [P][GRA_NXT]^3.  One CTA of 256 threads per patch; the GRA window is staged
-// in shared memory first.
+// in shared memory first.  Bound by memory (FP32, 4096 patches: 92 MB, within
+// L2), so it needs all its threads: two single cells each and eight CTAs per SM,
+// 12.7 us (FP64 35.3); runs of 16 bytes leave half of them without one in FP32
+// and take 40 registers: 16.8 us (FP64 41.8).
 template <typename T, int GG>
 __global__ void __launch_bounds__(256) gravity_kernel(T *__restrict__ flu, const T *__restrict__ pot,
                                                       int64_t npatch, T gra_const, int p5) {
