@@ -78,11 +78,14 @@ __device__ __forceinline__ double warp_sum(double v) {
 // Programmatic dependent launch: a kernel launched with launch_after() may become
 // resident while the kernel before it in the stream still runs.  pdl_wait() holds
 // it until that kernel has finished and its results are visible, before the first
-// access to global memory; pdl_trigger(), called by every CTA, says that the next
-// kernel may come in.  It is called when a CTA has only its results left to write:
-// earlier, the waiting CTAs took the places that freed first, and a launch smaller
-// than the device then ran unevenly spread (FP32 ghost 1, 1024 patches, back to
-// back: 14.4 us without, 19.7 triggered at the start, 12.9 before the output).
+// access to global memory.  Without pdl_trigger() the next kernel's CTAs come in
+// once all of this one's have ended, which still saves 2 us of a launch.
+// pdl_trigger() lets them in when every CTA of this kernel has called it or ended.
+// The SOR kernels don't: the waiting CTAs then crowd onto the SMs that are free
+// first, and a launch smaller than the device runs unevenly spread (FP64, back to
+// back, triggered before the output / not at all: ghost 1, 1001 patches 51.2 / 41.5
+// us, 2, 500 66.2 / 53.6, 4, 148 76.6 / 69.2, 5, 148 84.8 / 69.8; FP32 ghost 1,
+// 256 11.8 / 11.3, and 1 % in the mean of 85 launches).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 

@@ -561,11 +561,11 @@ struct SorLaneState {
 // potential and density come from `staged` in shared memory ([POT_NXT]^3
 // then [RHO_NXT]^3) instead of global memory.  PACK: FP32 two-row layouts
 // sweep in packed pairs (off where a solve takes about one sweep, which does not
-// pay for building them).  trigger: the patch is the CTA's last, see pdl_trigger().
+// pay for building them).
 template <typename T, int G, bool PHASED, int Z, int Y, bool STAGED = false, bool PACK = true, typename Hook>
 __device__ __forceinline__ void sor_solve_patch_with(const SolveArgs<T> &a, int64_t P_, int team, int tid,
                                                      unsigned char *tb, bool store, Hook &&hook,
-                                                     const T *staged = nullptr, bool trigger = false) {
+                                                     const T *staged = nullptr) {
   using g = Geo<G>;
   using C = SorCfg<T, G, Z, Y>;
   using S = SorSmem<T, G, Z, Y>;
@@ -775,15 +775,14 @@ __device__ __forceinline__ void sor_solve_patch_with(const SolveArgs<T> &a, int6
     if (a.resid) a.resid[P_] = last;
   }
 
-  if (trigger) pdl_trigger();
   // ---- output window and fused gravity update ------------------------------
   patch_output<T, G, TEAM>(a, P_, tid, [s_cube](int x, int y, int z) GPG_INLINE { return s_cube[C::addr(x, y, z)]; });
 }
 
 template <typename T, int G, bool PHASED, int Z = 1, int Y = 1>
 __device__ __forceinline__ void sor_solve_patch(const SolveArgs<T> &a, int64_t P_, int team, int tid,
-                                                unsigned char *tb, bool trigger = false) {
-  sor_solve_patch_with<T, G, PHASED, Z, Y>(a, P_, team, tid, tb, true, [](const auto &) {}, nullptr, trigger);
+                                                unsigned char *tb) {
+  sor_solve_patch_with<T, G, PHASED, Z, Y>(a, P_, team, tid, tb, true, [](const auto &) {});
 }
 
 // PPC: teams (patches) per CTA.  PHASED: form the MH independent updates of a
@@ -802,7 +801,7 @@ __global__ void __launch_bounds__(PPC *SorCfg<T, G, Z, Y>::TEAM)
   const int64_t P_ = int64_t(blockIdx.x) * PPC + team;
   pdl_wait();
   if (P_ >= a.npatch) return;  // whole team leaves together
-  sor_solve_patch<T, G, PHASED, Z, Y>(a, P_, team, tid, smem_raw + team * SorSmem<T, G, Z, Y>::team_bytes, true);
+  sor_solve_patch<T, G, PHASED, Z, Y>(a, P_, team, tid, smem_raw + team * SorSmem<T, G, Z, Y>::team_bytes);
 }
 
 // ---------------------------------------------------------------------------
@@ -867,7 +866,7 @@ __global__ void __launch_bounds__(TPC *SorCfg<T, G, Z, Y>::TEAM, (StagedSmem<T, 
             stage(next);
           }
         },
-        stg, next >= a.npatch);
+        stg);
     if (!arrived && tid == 0) {
       if (a.iters) a.iters[P_] = -1;
       if (a.resid) a.resid[P_] = __longlong_as_double(0x7ff8000000000000ll);
