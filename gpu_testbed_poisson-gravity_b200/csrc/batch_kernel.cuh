@@ -57,7 +57,7 @@ __device__ __forceinline__ void batch_unit(const SolveArgs<T> &a, int64_t unit_i
   const int64_t P = unit_in_group * U::TEAMS + team;
   if (P >= a.npatch) return;     // last unit of a group may be partial
   using L = BatchLayout<T>;
-  sor_solve_patch<T, G, false, L::Z, L::Y>(a, P, team, tid, smem + team * U::team_bytes);
+  sor_solve_patch<T, G, false, L::Z, L::Y, true>(a, P, team, tid, smem + team * U::team_bytes);
 }
 
 // Resident CTAs per SM the register allocation must allow (the five ghost

@@ -101,14 +101,16 @@ __device__ __forceinline__ void gravity_patch(T *__restrict__ flu, int tid, T gr
 
 // What every solver kernel leaves of a patch: the GRA_NXT^3 window of the solved
 // cube (CPU_PoissonSolver_SOR.cpp:305-311) and, with gra_acc, the updated fluid.
-// cube(x, y, z) reads the solver's cube.  The first fluid loads are under way
-// while the window is written.
-template <typename T, int G, int NT, typename Cube>
+// cube(x, y, z) reads the solver's cube.  PRELOAD: the first fluid loads are under
+// way while the window is written, at the price of their registers (20 in FP32,
+// 20 to 40 in FP64) over the window's address arithmetic; the callers say where
+// that pays.  CELLS: see FluidRun.
+template <typename T, int G, int NT, bool PRELOAD = true, int CELLS = 16 / sizeof(T), typename Cube>
 __device__ __forceinline__ void patch_output(const SolveArgs<T> &a, int64_t P, int tid, Cube cube) {
   T *flu = a.flu + P * 5 * 512;
   const bool al = aligned16(flu);
-  FluidRun<T> f;
-  if (a.gra_acc && tid < FluidRun<T>::RUNS) f.load(flu, tid, al);
+  FluidRun<T, CELLS> f;
+  if (PRELOAD && a.gra_acc && tid < FluidRun<T, CELLS>::RUNS) f.load(flu, tid, al);
   // (edge GN a compile-time constant per GRA_GHOST_SIZE: the index split is
   // then multiply-shift, not division)
   auto window = [&](auto gg) {
@@ -128,8 +130,8 @@ __device__ __forceinline__ void patch_output(const SolveArgs<T> &a, int64_t P, i
   // fused gravity update (CPU_GravitySolver.cpp:34-79)
   if (a.gra_acc) {
     auto phi = [&](int i, int j, int k) { return cube(i + G, j + G, k + G); };
-    for (int run = tid; run < FluidRun<T>::RUNS; run += NT) {
-      if (run >= NT) f.load(flu, run, al);
+    for (int run = tid; run < FluidRun<T, CELLS>::RUNS; run += NT) {
+      if (!PRELOAD || run >= NT) f.load(flu, run, al);
       f.update(run, a.gra_const, a.p5, phi);
       f.store(flu, run, al);
     }

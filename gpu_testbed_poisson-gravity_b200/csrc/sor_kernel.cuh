@@ -561,8 +561,9 @@ struct SorLaneState {
 // potential and density come from `staged` in shared memory ([POT_NXT]^3
 // then [RHO_NXT]^3) instead of global memory.  PACK: FP32 two-row layouts
 // sweep in packed pairs (off where a solve takes about one sweep, which does not
-// pay for building them).
-template <typename T, int G, bool PHASED, int Z, int Y, bool STAGED = false, bool PACK = true, typename Hook>
+// pay for building them).  QUEUE: one of the ghost sizes of the work-queue kernel.
+template <typename T, int G, bool PHASED, int Z, int Y, bool STAGED = false, bool PACK = true, bool QUEUE = false,
+          typename Hook>
 __device__ __forceinline__ void sor_solve_patch_with(const SolveArgs<T> &a, int64_t P_, int team, int tid,
                                                      unsigned char *tb, bool store, Hook &&hook,
                                                      const T *staged = nullptr) {
@@ -776,13 +777,23 @@ __device__ __forceinline__ void sor_solve_patch_with(const SolveArgs<T> &a, int6
   }
 
   // ---- output window and fused gravity update ------------------------------
-  patch_output<T, G, TEAM>(a, P_, tid, [s_cube](int x, int y, int z) GPG_INLINE { return s_cube[C::addr(x, y, z)]; });
+  // The fluid is loaded ahead where its registers are to be had: in FP32 outside
+  // the staged and work-queue kernels, whose loops spilled for it (FP32 work queue
+  // 1164 bytes of spill stores, 184 without), and in FP64 in the staged ghost 5
+  // alone (4096 patches 1234 us, 1275 without, 1282 before; the FP64 queue spilled
+  // 1564 bytes: 20001 patches 5304 us, 3644 without; staged ghost 2, 1001 patches
+  // 121 / 94).  One-row FP64 lanes take single cells (ghost 4, split columns, 1001
+  // patches: 346 us, 413 with runs of two, which the allocator pays for in the sweeps).
+  constexpr bool F64 = sizeof(T) == 8;
+  constexpr bool PRELOAD = F64 ? STAGED && G == 5 : !STAGED && !QUEUE;
+  constexpr int CELLS = F64 && Y == 1 ? 1 : 16 / int(sizeof(T));
+  patch_output<T, G, TEAM, PRELOAD, CELLS>(a, P_, tid, [s_cube](int x, int y, int z) GPG_INLINE { return s_cube[C::addr(x, y, z)]; });
 }
 
-template <typename T, int G, bool PHASED, int Z = 1, int Y = 1>
+template <typename T, int G, bool PHASED, int Z = 1, int Y = 1, bool QUEUE = false>
 __device__ __forceinline__ void sor_solve_patch(const SolveArgs<T> &a, int64_t P_, int team, int tid,
                                                 unsigned char *tb) {
-  sor_solve_patch_with<T, G, PHASED, Z, Y>(a, P_, team, tid, tb, true, [](const auto &) {});
+  sor_solve_patch_with<T, G, PHASED, Z, Y, false, true, QUEUE>(a, P_, team, tid, tb, true, [](const auto &) {});
 }
 
 // PPC: teams (patches) per CTA.  PHASED: form the MH independent updates of a

@@ -13,6 +13,13 @@ LIB = os.path.join(REPO, "gpu_testbed_poisson-gravity_b200", "lib", "libgpg.so")
 LIMITS = [
     ("14gravity_kernelIfLi1EE", 32, 0),     # eight CTAs of 256 threads per SM
     ("14gravity_kernelIfLi2EE", 32, 0),
+    ("16sor_batch_kernelIfE", 128, 500),    # three and four CTAs per SM, bounded so
+    ("16sor_batch_kernelIdE", 168, 500),
+    ("17staged_sor_kernelIfLi2ELb1ELi2ELi2ELi2EE", 96, 50),
+    ("17staged_sor_kernelIfLi3ELb1ELi2ELi2ELi1EE", 96, 0),
+    ("17staged_sor_kernelIdLi3ELb1ELi2ELi2ELi1EE", 168, 50),
+    ("17staged_sor_kernelIdLi4ELb0ELi2ELi2ELi1EE", 255, 0),
+    ("10sor_kernelIdLi4ELi1ELb1ELi2ELi1EE", 128, 0),
 ]
 
 
