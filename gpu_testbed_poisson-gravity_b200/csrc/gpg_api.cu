@@ -126,8 +126,9 @@ std::atomic<bool> g_sor_pinned[2][6] = {};
 // large-launch layout at every size, ghost 4 the split column up to 1024 (45.6
 // us; the whole one 45.8, at 256 patches 20.6 and 22.7) and, with one patch per SM,
 // one row per lane (64 patches 14.5 -> 12.1, 100 16.5 -> 14.0; 200 18.6 -> 18.9).
-// FP64 ghost 2 at 256 53.6 -> 39.1, ghost 4 the staged kernel while half the SMs
-// have a patch (64: 65.7 -> 60.3; 150: 79.0 -> 81.0).  FP64 ghost 5 keeps the
+// FP64 ghost 2 at 256 53.6 -> 39.1, ghost 4 the staged kernel while each of its teams,
+// two per SM, has one patch (64 patches 67.1 -> 57.4, 148 68.6 -> 59.0, 296 85.8 ->
+// 81.5; 370 113 and 128).  FP64 ghost 5 keeps the
 // unstaged v11 up to 1024 patches: the staged kernel hands patches out at a
 // fixed stride, and 1024 patches over its 296 teams leave some teams a fourth
 // patch (333 vs 360 us; through the CUAPI path, 4 streams of 1024 patches,
@@ -138,7 +139,7 @@ struct SorSmall {
 constexpr SorSmall kSorSmall[2][6][2] = {
     // ghost 0 (none), 1, 2, 3, 4, 5; the smaller limit first, 0 none
     {{}, {{2048, 7}}, {{512, 6}}, {{512, 7}}, {{148, 6}, {1024, 11}}, {}},  // float
-    {{}, {{256, 8}}, {{256, 7}}, {}, {{74, 15}}, {{1024, 11}}},             // double
+    {{}, {{256, 8}}, {{256, 7}}, {}, {{296, 14}}, {{1024, 11}}},            // double
 };
 std::once_flag g_tune_once;
 
