@@ -625,30 +625,45 @@ __device__ __forceinline__ void sor_solve_patch_with(const SolveArgs<T> &a, int6
     // start's kernel was slower with pairs (65536 patches 294 us, 299 with)
     const T *rho = STAGED ? staged + g::PN3 : a.rho + P_ * g::RHO3;
     const bool pairs = (reinterpret_cast<uintptr_t>(rho) & 7) == 0;
+    auto columns = [&](auto fetch) GPG_INLINE {
 #pragma unroll
-    for (int rr = 0; rr < Y; ++rr) {
-      const int yr = y + rr;
+      for (int rr = 0; rr < Y; ++rr) {
+        const int yr = y + rr;
 #pragma unroll
-      for (int zz = 1; zz <= MH; ++zz) {
-        const int z = zbase + zz;
-        const T *q = rho + ((z - 1) * M + (yr - 1)) * M + 2 * h;
+        for (int zz = 1; zz <= MH; ++zz) {
+          const int z = zbase + zz;
+          const float2 rv = fetch(rho + ((z - 1) * M + (yr - 1)) * M + 2 * h);
+          const bool left0 = ((yr + z) & 1) == 0;  // colour 0 is the left cell
+          crho[rr][0][zz - 1] = active ? mul(a.sor_const, left0 ? rv.x : rv.y) : T(0);
+          crho[rr][1][zz - 1] = active ? mul(a.sor_const, left0 ? rv.y : rv.x) : T(0);
+        }
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+          for (int zz = 0; zz < MH + 2; ++zz) v[rr][c][zz] = s_cube[(c * N + zbase + zz) * PP + ln.own + rr * P];
+      }
+    };
+    auto one = [](const T *q) GPG_INLINE { return make_float2(q[0], q[1]); };
+    auto two = [](const T *q) GPG_INLINE { return __ldg(reinterpret_cast<const float2 *>(q)); };
+    if constexpr (!STAGED && Z == 1 && Y == 1) {
+      // one row, a whole column: one branch around all loads, which then are in
+      // flight together (variant 0, ghost 3, 148 patches: 24.1 -> 15.2 us).  The split
+      // one-row layout is slower so (ghost 4, 64 patches 13.1 / 14.6)
+      if (pairs)
+        columns(two);
+      else
+        columns(one);
+    } else {
+      columns([&](const T *q) GPG_INLINE {
         float2 rv = make_float2(0.f, 0.f);
         if (active) {
-          if (!STAGED && pairs) {
-            rv = __ldg(reinterpret_cast<const float2 *>(q));
-          } else {
-            rv.x = q[0];
-            rv.y = q[1];
-          }
+          if (!STAGED && pairs)
+            rv = two(q);
+          else
+            rv = one(q);
         }
-        const bool left0 = ((yr + z) & 1) == 0;  // colour 0 is the left cell
-        crho[rr][0][zz - 1] = active ? mul(a.sor_const, left0 ? rv.x : rv.y) : T(0);
-        crho[rr][1][zz - 1] = active ? mul(a.sor_const, left0 ? rv.y : rv.x) : T(0);
-      }
-#pragma unroll
-      for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int zz = 0; zz < MH + 2; ++zz) v[rr][c][zz] = s_cube[(c * N + zbase + zz) * PP + ln.own + rr * P];
+        return rv;
+      });
     }
     // tolerance scale: sum |Const rho| (mode 1) or sum |interpolated phi| over the
     // updated cells, before a start mode replaces it (3)

@@ -40,3 +40,32 @@ def test_overlapped_solves(g, npatch):
     for k in range(22):
         best[k & 1] = min(best[k & 1], us(k & 1))
     assert best[0] <= 1.04 * best[1]
+
+
+def test_one_row_layouts_load_together():
+    """FP32, one row and a whole column per lane: the pass by heights (variant 0) and
+    the phased one (1) set up alike; a serial chain of loads made the first 1.4
+    times as slow as the second (1.04 without it)."""
+    torch = pytest.importorskip("torch")
+    from gpg.lib import check, library, solve_device
+    n, g = 148, 3
+    d = make_patches(n, g, seed=3)
+    rho, pin, flu = (torch.from_numpy(d[k]).cuda() for k in ("rho", "pot_in", "flu"))
+    p = default_params(4, g, GPG_SOR)
+    out = torch.empty((n, 10, 10, 10), device="cuda")
+    iters = torch.empty(n, device="cuda", dtype=torch.int32)
+    resid = torch.empty(n, device="cuda", dtype=torch.float64)
+    best = [1e9, 1e9]
+    try:
+        for k in range(22):
+            check(library().gpg_set_sor_variant(4, g, k & 1))
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            e0.record()
+            for _ in range(40):
+                solve_device(p, rho, pin, pot_out=out, flu=flu, iters=iters, resid=resid)
+            e1.record()
+            e1.synchronize()
+            best[k & 1] = min(best[k & 1], e0.elapsed_time(e1) * 25)
+    finally:
+        check(library().gpg_set_sor_variant(4, g, -1))
+    assert best[0] <= 1.2 * best[1]

@@ -72,3 +72,29 @@ def test_wide_loads_fall_back_off_their_alignment(rs, g, gg, scheme):
         got = solve_device(p, off(t["rho"], k), off(t["pot_in"], k), flu=off(t["flu"], k))
         for a, b in zip(got, want):
             assert torch.equal(a, b), k
+
+
+@pytest.mark.parametrize("g", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("init", [0, 1])
+def test_one_row_columns_off_their_alignment(g, init):
+    """FP32 lanes of one row and a whole column choose between pair and single
+    density loads once for the column: the same bits either way."""
+    torch = pytest.importorskip("torch")
+    from gpg.lib import check, library, solve_device
+    d = make_patches(37, g, seed=80 + g, dtype=np.float32, fluid=False)
+    rho, pin = (torch.from_numpy(d[k]).cuda() for k in ("rho", "pot_in"))
+    buf = torch.empty(rho.numel() + 1, device="cuda")
+    buf[1:] = rho.reshape(-1)
+    p = default_params(4, g, GPG_SOR, gra_acc=0, init_mode=init)
+    try:
+        for v in range(6):
+            check(library().gpg_set_sor_variant(4, g, v))
+            try:
+                want = solve_device(p, rho, pin)
+            except Exception:       # more threads than the registers allow
+                continue
+            got = solve_device(p, buf[1:].view(rho.shape), pin)
+            for k in (0, 2, 3):
+                assert torch.equal(got[k], want[k]), v
+    finally:
+        check(library().gpg_set_sor_variant(4, g, -1))
