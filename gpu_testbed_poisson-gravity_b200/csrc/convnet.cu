@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "../../include/gpg.h"
+#include "arena.cuh"
 #include "args.cuh"
 #include "common.cuh"
 #include "convnet_kernels.cuh"
@@ -297,6 +298,7 @@ struct gpg_net {
   int max_batch = 0;
   int probe_polls = 0;  // test hook of the inference kernel (gpg_net_set_wait_probe)
   int64_t step = 0;
+  void *block = nullptr;  // holds all arrays below
   float *params = nullptr, *grad = nullptr, *adam_m = nullptr, *adam_v = nullptr;
   __nv_bfloat16 *wf0 = nullptr, *wf3[kLayers] = {}, *wb3[kLayers] = {};
   // planes: input, activations (each replaced by its gradient on the way back), loss gradient
@@ -394,27 +396,7 @@ int gradients(gpg_net *n, int64_t npatch, const float *rho, const float *pot_in,
   return GPG_OK;
 }
 
-void free_net(gpg_net *n) {
-  cudaFree(n->params);
-  cudaFree(n->grad);
-  cudaFree(n->adam_m);
-  cudaFree(n->adam_v);
-  for (int l = 0; l < kLayers; ++l) {
-    cudaFree(n->wf3[l]);
-    cudaFree(n->wb3[l]);
-  }
-  cudaFree(n->x0);
-  for (auto *p : n->act) cudaFree(p);
-  cudaFree(n->wf0);
-  cudaFree(n->g4);
-  cudaFree(n->scale);
-  for (int l = 0; l < kLayers; ++l) {
-    cudaFree(n->wpart[l]);
-    cudaFree(n->bpart[l]);
-  }
-  cudaFree(n->loss_part);
-  cudaFree(n->err);
-}
+void free_net(gpg_net *n) { cudaFree(n->block); }
 
 }  // namespace
 
@@ -431,42 +413,37 @@ extern "C" int gpg_net_create(gpg_net **out, int max_batch, uint64_t seed, int d
   *out = nullptr;
   if (max_batch < 1 || max_batch > (1 << 20)) return nfail(GPG_ERR_INVALID, "max_batch %d", max_batch);
   NET_CUDA(cudaSetDevice(device_id));
-  cudaDeviceProp prop;
-  NET_CUDA(cudaGetDeviceProperties(&prop, device_id));
-  if (prop.major != 10) return nfail(GPG_ERR_UNSUPPORTED, "tensor-core kernels need sm_100 (found sm_%d%d)",
-                                     prop.major, prop.minor);
+  int major = 0, minor = 0;
+  NET_CUDA(gpg::compute_capability(device_id, &major, &minor));
+  if (major != 10) return nfail(GPG_ERR_UNSUPPORTED, "tensor-core kernels need sm_100 (found sm_%d%d)", major, minor);
   auto *n = new gpg_net;
   n->device = device_id;
   n->max_batch = max_batch;
-  cudaError_t e = cudaSuccess;
-  auto al = [&](void **p, size_t b) {
-    if (e == cudaSuccess) e = cudaMalloc(p, b);
-    if (e == cudaSuccess) e = cudaMemset(*p, 0, b);
-  };
-  al((void **)&n->params, kParams * 4);
-  al((void **)&n->grad, kParams * 4);
-  al((void **)&n->adam_m, kParams * 4);
-  al((void **)&n->adam_v, kParams * 4);
-  for (int l = 0; l < kLayers; ++l) {
-    if (l == 0) {
-      al((void **)&n->wf0, size_t(KChunks<kCin[0]>::KCH) * kCout[0] * 16);
-    } else {
-      al((void **)&n->wf3[l], size_t(w_count(l)) * 2);
-      al((void **)&n->wb3[l], size_t(w_count(l)) * 2);
-    }
+  gpg::Arena arena;
+  arena.add(n->err, 1);
+  arena.add(n->params, kParams);
+  arena.add(n->grad, kParams);
+  arena.add(n->adam_m, kParams);
+  arena.add(n->adam_v, kParams);
+  // the kernels write cells only, the planes' other rows stay zero
+  arena.add(n->x0, size_t(max_batch) * plane_elems(8));
+  for (auto &p : n->act) arena.add(p, size_t(max_batch) * plane_elems(32));
+  arena.add(n->g4, size_t(max_batch) * plane_elems(16));
+  arena.zeroed_to_here();
+  arena.add(n->wf0, size_t(KChunks<kCin[0]>::KCH) * kCout[0] * 8);
+  for (int l = 1; l < kLayers; ++l) {
+    arena.add(n->wf3[l], size_t(w_count(l)));
+    arena.add(n->wb3[l], size_t(w_count(l)));
   }
-  // zero-filled: the kernels write cells only, the planes' other rows stay zero
-  al((void **)&n->x0, size_t(max_batch) * plane_elems(8) * 2);
-  for (auto &p : n->act) al((void **)&p, size_t(max_batch) * plane_elems(32) * 2);
-  al((void **)&n->g4, size_t(max_batch) * plane_elems(16) * 2);
-  al((void **)&n->scale, size_t(max_batch) * 4);
-  const size_t ctas = sm_count();  // one per SM at most
+  arena.add(n->scale, size_t(max_batch));
+  // partial sums of the CTAs: one per SM at most, and no more than there are planes
+  const size_t ctas = std::min<size_t>(size_t(max_batch) * kEdge, sm_count());
   for (int l = 0; l < kLayers; ++l) {
-    al((void **)&n->wpart[l], ctas * 27 * kCin[l] * (l == 3 ? 1 : 32) * 4);
-    al((void **)&n->bpart[l], ctas * 32 * 4);
+    arena.add(n->wpart[l], ctas * 27 * kCin[l] * (l == 3 ? 1 : 32));
+    arena.add(n->bpart[l], ctas * 32);
   }
-  al((void **)&n->loss_part, ctas * 8);
-  al((void **)&n->err, 4);
+  arena.add(n->loss_part, ctas);
+  cudaError_t e = arena.allocate(&n->block);
   if (e != cudaSuccess) {
     free_net(n);
     delete n;

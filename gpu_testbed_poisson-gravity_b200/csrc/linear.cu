@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "../../include/gpg.h"
+#include "arena.cuh"
 #include "args.cuh"
 #include "lin_sor.cuh"
 #include "optim.cuh"
@@ -103,6 +104,7 @@ __global__ void lin_adam_kernel(const gpg::AdamArgs a, __nv_bfloat16 *__restrict
 constexpr int kGradSplit = 37;               // CTAs that share a block's patches
 constexpr int kChunk = 64;                   // patches per step
 constexpr int kGradThreads = 256;
+inline int grad_splits(int npatch) { return std::min(kGradSplit, (npatch + kChunk - 1) / kChunk); }
 constexpr int kPitchW = kK + 4;              // row pitches (words) that keep the 128-bit accesses aligned
 struct GradSmem {
   float wt[kK][kPitchW];                     // W[c]^T: [k][row]
@@ -249,6 +251,7 @@ struct gpg_lin {
   int max_batch = 0;
   int step = 0;
   int probe_polls = 0;
+  void *block = nullptr;  // holds all arrays below
   float *params = nullptr, *grad = nullptr, *adam_m = nullptr, *adam_v = nullptr;
   float *part = nullptr, *loss = nullptr;  // partial gradients [kGradSplit * 8][64][64]
   double *loss_part = nullptr;
@@ -320,30 +323,25 @@ extern "C" int gpg_lin_create(gpg_lin **out, int max_batch, int device_id) {
   if (cudaGetDeviceCount(&count) != cudaSuccess || device_id < 0 || device_id >= count)
     return lfail(GPG_ERR_NO_DEVICE, "device %d of %d", device_id, count);
   LIN_CUDA(cudaSetDevice(device_id));
-  cudaDeviceProp prop;
-  LIN_CUDA(cudaGetDeviceProperties(&prop, device_id));
-  if (prop.major != 10)
-    return lfail(GPG_ERR_UNSUPPORTED, "tensor-core kernels need sm_100 (found sm_%d%d)", prop.major, prop.minor);
+  int major = 0, minor = 0;
+  LIN_CUDA(gpg::compute_capability(device_id, &major, &minor));
+  if (major != 10) return lfail(GPG_ERR_UNSUPPORTED, "tensor-core kernels need sm_100 (found sm_%d%d)", major, minor);
   gpg_lin *l = new gpg_lin;
   l->device = device_id;
   l->max_batch = max_batch;
-  cudaError_t e = cudaSuccess;
-  auto al = [&](void **p, size_t bytes) {
-    if (e == cudaSuccess) e = cudaMalloc(p, bytes);
-  };
-  al((void **)&l->params, kParams * 4);
-  al((void **)&l->grad, kParams * 4);
-  al((void **)&l->adam_m, kParams * 4);
-  al((void **)&l->adam_v, kParams * 4);
-  al((void **)&l->tiles, 2 * gpg::lin::kTileBytes);
-  al((void **)&l->part, size_t(kGradSplit) * 8 * kK * kK * 4);
-  al((void **)&l->loss_part, size_t(kGradSplit) * 8 * 8);
-  al((void **)&l->loss, 4);
-  al((void **)&l->err, 4);
-  if (e == cudaSuccess) e = cudaMemset(l->params, 0, kParams * 4);
-  if (e == cudaSuccess) e = cudaMemset(l->adam_m, 0, kParams * 4);
-  if (e == cudaSuccess) e = cudaMemset(l->adam_v, 0, kParams * 4);
-  if (e == cudaSuccess) e = cudaMemset(l->err, 0, 4);
+  gpg::Arena arena;
+  arena.add(l->err, 1);
+  arena.add(l->params, kParams);
+  arena.add(l->adam_m, kParams);
+  arena.add(l->adam_v, kParams);
+  arena.zeroed_to_here();
+  arena.add(l->grad, kParams);
+  arena.add(l->tiles, gpg::lin::kTileBytes);  // two tiles of 2-byte values
+  const size_t splits = grad_splits(max_batch);
+  arena.add(l->part, splits * 8 * kK * kK);
+  arena.add(l->loss_part, splits * 8);
+  arena.add(l->loss, 1);
+  cudaError_t e = arena.allocate(&l->block);
   if (e != cudaSuccess) {
     gpg_lin_destroy(l);
     return lfail(e == cudaErrorMemoryAllocation ? GPG_ERR_OOM : GPG_ERR_CUDA, "allocation: %s", cudaGetErrorString(e));
@@ -371,9 +369,7 @@ extern "C" int gpg_lin_create(gpg_lin **out, int max_batch, int device_id) {
 extern "C" int gpg_lin_destroy(gpg_lin *l) {
   if (!l) return GPG_OK;
   cudaSetDevice(l->device);
-  for (void *p : {(void *)l->params, (void *)l->grad, (void *)l->adam_m, (void *)l->adam_v, (void *)l->tiles,
-                  (void *)l->part, (void *)l->loss_part, (void *)l->loss, (void *)l->err})
-    cudaFree(p);
+  cudaFree(l->block);
   delete l;
   return GPG_OK;
 }
@@ -466,7 +462,7 @@ extern "C" int gpg_lin_gradients(gpg_lin *l, int npatch, const float *d_u, const
   if (!d_u || !d_t) return lfail(GPG_ERR_INVALID, "NULL array");
   LIN_CUDA(cudaSetDevice(l->device));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int nsplit = std::min(kGradSplit, (npatch + kChunk - 1) / kChunk);
+  const int nsplit = grad_splits(npatch);
   LIN_CUDA(gpg::launch_after(lin_grad_kernel, dim3(8, nsplit), kGradThreads, sizeof(GradSmem), s, d_u, d_t, l->params,
                              npatch, l->part, l->loss_part));
   LIN_CUDA(gpg::launch_after(lin_reduce_kernel, kParams / 64, 256, 0, s, l->part, l->loss_part, nsplit, npatch,
