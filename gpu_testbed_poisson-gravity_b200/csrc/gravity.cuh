@@ -48,7 +48,7 @@ __device__ __forceinline__ void gravity_cell(int i, int j, int k, T gra_const, i
 template <typename T, int CELLS = 16 / sizeof(T)>
 struct FluidRun {
   static constexpr int W = CELLS, RUNS = 512 / W;
-  T q[5][W];  // component, cell
+  alignas(16) T q[5][W];  // component, cell; a row is one wide access
   __device__ __forceinline__ void load(const T *flu, int run, bool aligned) {
 #pragma unroll
     for (int c = 0; c < 5; ++c) {

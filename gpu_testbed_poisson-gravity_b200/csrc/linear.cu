@@ -159,8 +159,10 @@ __global__ void __launch_bounds__(kGradThreads) lin_grad_kernel(const float *__r
     for (int k = 0; k < kK; k += 4) {
       float x[4][4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        *reinterpret_cast<float4 *>(x[q]) = *reinterpret_cast<const float4 *>(&sm.u[p0 + q][k]);
+      for (int q = 0; q < 4; ++q) {
+        const float4 uk = *reinterpret_cast<const float4 *>(&sm.u[p0 + q][k]);
+        x[q][0] = uk.x, x[q][1] = uk.y, x[q][2] = uk.z, x[q][3] = uk.w;
+      }
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
         const float4 wk = *reinterpret_cast<const float4 *>(&sm.wt[k + kk][r0]);
