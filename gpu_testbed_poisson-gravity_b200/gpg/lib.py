@@ -100,10 +100,13 @@ def stream_ptr(stream, device_index: int) -> int:
     """Handle of `stream` (a torch.cuda.Stream), or of the device's current
     stream when None.  The raw handle is read without building a Stream object:
     a small solve's launch is otherwise shorter than the call around it (256
-    patches at ghost 1: 10.8 us a call on the host before, 9.7 now)."""
+    patches at ghost 1: 10.8 us a call on the host before, 9.7 now); the function
+    for it is not public, so a torch without it goes through the object."""
     if stream is not None:
         return stream.cuda_stream
-    return torch_module()._C._cuda_getCurrentRawStream(device_index)
+    torch = torch_module()
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return torch.cuda.current_stream(device_index).cuda_stream if raw is None else raw(device_index)
 
 
 _torch = None
