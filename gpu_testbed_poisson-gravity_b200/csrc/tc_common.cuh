@@ -63,29 +63,10 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n, bool a_mn, bool 
          (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 
-// D(tmem) = A * B (+ D when accumulate), issued by one thread
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                         uint32_t accumulate) {
-  const uint32_t zero = 0;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}\n" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(zero)
-      : "memory");
-}
-
-// the mbarrier at `bar` receives one arrival when every MMA issued so far by
-// this thread has completed
-__device__ __forceinline__ void mma_commit(uint64_t *bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-
-// The same two, executed by a whole converged warp with warp-uniform operands,
-// one elected lane issuing.  Descriptors then stay in uniform registers: from a
-// single-lane branch every MMA with a descriptor of its own takes 81 cycles,
-// this way 43 (M 128, N 32: the operand reads' own time).
+// D(tmem) = A * B (+ D when accumulate), executed by a whole converged warp with
+// warp-uniform operands, one elected lane issuing.  Descriptors then stay in
+// uniform registers: from a single-lane branch every MMA with a descriptor of its
+// own takes 81 cycles, this way 43 (M 128, N 32: the operand reads' own time).
 __device__ __forceinline__ void mma_bf16_warp(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                               uint32_t accumulate) {
   const uint32_t zero = 0;
@@ -97,6 +78,8 @@ __device__ __forceinline__ void mma_bf16_warp(uint32_t d_tmem, uint64_t a_desc, 
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(zero)
       : "memory");
 }
+// the mbarrier at `bar` receives one arrival when every MMA issued so far by this
+// warp's elected lane has completed (the same lane each time); by a whole warp
 __device__ __forceinline__ void mma_commit_warp(uint64_t *bar) {
   asm volatile(
       "{\n\t.reg .pred q;\n\t"
