@@ -57,10 +57,11 @@ LIN_FLOP_EXECUTED = 16 * 2 * 128 * 16 * 16 // 8
 # algorithmic FLOPs of one patch's forward pass: 3^3 convolutions 3 -> 32 -> 32
 # -> 32 on the 10^3 cube, 32 -> 1 on the 8^3 interior
 NET_FLOP = 2 * 27 * (1000 * (3 * 32 + 32 * 32 + 32 * 32) + 512 * 32)
-# FLOPs the fused kernel's MMAs execute per patch (M=128 x K=16 tiles): 10 row
-# tiles x 14 tap pairs (N=32) for layer 1, 10 x 27 x 2 K halves (N=32) for
-# layers 2 and 3, 8 x 27 x 2 (N=16) for layer 4
-NET_FLOP_EXECUTED = 2 * 128 * 16 * (32 * (10 * 14 + 2 * 10 * 27 * 2) + 16 * 8 * 27 * 2)
+# FLOPs the fused kernel's MMAs execute per patch (M=128 x K=16 tiles): 10 planes
+# x 14 tap pairs (N=32) for layer 1; a plane's window adds to up to three output
+# planes at once, 18 MMAs of N = 32 per plane for layers 2 and 3 (28 of the 30
+# exist) and of N = 16 for layer 4 (24, interior planes alone)
+NET_FLOP_EXECUTED = 2 * 128 * 16 * (32 * 10 * 14 + 2 * 18 * 32 * 28 + 18 * 16 * 24)
 
 
 def dataset(n: int, seed: int, dtype=np.float32, first: int = 0, stop: int | None = None):
