@@ -105,8 +105,10 @@ def stream_ptr(stream, device_index: int) -> int:
     if stream is not None:
         return stream.cuda_stream
     torch = torch_module()
-    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-    return torch.cuda.current_stream(device_index).cuda_stream if raw is None else raw(device_index)
+    try:
+        return torch._C._cuda_getCurrentRawStream(device_index)
+    except AttributeError:
+        return torch.cuda.current_stream(device_index).cuda_stream
 
 
 _torch = None
