@@ -793,14 +793,16 @@ __device__ __forceinline__ void sor_solve_patch_with(const SolveArgs<T> &a, int6
 
   // ---- output window and fused gravity update ------------------------------
   // The fluid is loaded ahead where its registers are to be had: in FP32 outside
-  // the staged and work-queue kernels, whose loops spilled for it (FP32 work queue
-  // 1164 bytes of spill stores, 184 without), and in FP64 in the staged ghost 5
-  // alone (4096 patches 1234 us, 1275 without, 1282 before; the FP64 queue spilled
-  // 1564 bytes: 20001 patches 5304 us, 3644 without; staged ghost 2, 1001 patches
-  // 121 / 94).  One-row FP64 lanes take single cells (ghost 4, split columns, 1001
-  // patches: 346 us, 413 with runs of two, which the allocator pays for in the sweeps).
+  // the packed staged kernels and the work queue, whose loops spilled for it (FP32
+  // work queue 1164 bytes of spill stores, 184 without; the learned start's kernel
+  // gains: 65536 patches with gravity 557 us, 567 without), and in FP64 in the staged
+  // ghost 5 alone (4096 patches 1234 us, 1275 without, 1282 before; the FP64 queue
+  // spilled 1564 bytes: 20001 patches 5304 us, 3644 without; staged ghost 2, 1001
+  // patches 121 / 94).  One-row FP64 lanes take single cells (ghost 4, split columns,
+  // 1001 patches: 346 us, 413 with runs of two, which the allocator pays for in the
+  // sweeps).
   constexpr bool F64 = sizeof(T) == 8;
-  constexpr bool PRELOAD = F64 ? STAGED && G == 5 : !STAGED && !QUEUE;
+  constexpr bool PRELOAD = F64 ? STAGED && G == 5 : (!STAGED || !PACK) && !QUEUE;
   constexpr int CELLS = F64 && Y == 1 ? 1 : 16 / int(sizeof(T));
   patch_output<T, G, TEAM, PRELOAD, CELLS>(a, P_, tid, [s_cube](int x, int y, int z) GPG_INLINE { return s_cube[C::addr(x, y, z)]; });
 }
