@@ -10,9 +10,9 @@
 namespace gpg {
 
 // Launch `fn`, which begins with pdl_wait(), so that its start overlaps the end
-// of the kernel before it in the stream (common.cuh): 1 to 2 us of a back-to-back
-// launch, 7-15 % of a small solve (FP32 ghost 1, 256 patches 12.4 -> 11.3 us;
-// ghost 3 18.5 -> 15.9).
+// of the kernel before it in the stream (common.cuh): about 2 us of a back-to-back
+// launch (FP32 ghost 1, 256 patches 12.4 -> 10.2 us; FP64 ghost 2, 500 patches 55.9 ->
+// 53.6).
 template <typename... Params, typename... Args>
 inline cudaError_t launch_after(void (*fn)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                                 Args... args) {

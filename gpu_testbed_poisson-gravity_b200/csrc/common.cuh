@@ -86,6 +86,12 @@ __device__ __forceinline__ double warp_sum(double v) {
 // back, triggered before the output / not at all: ghost 1, 1001 patches 51.2 / 41.5
 // us, 2, 500 66.2 / 53.6, 4, 148 76.6 / 69.2, 5, 148 84.8 / 69.8; FP32 ghost 1,
 // 256 11.8 / 11.3, and 1 % in the mean of 85 launches).
+// The others do: multigrid before its output (FP64 ghost 2, 148 patches 77.7 us, 79.8
+// without; ghost 1, 500 69.5 / 63.2), the learned start's kernel after its last
+// patch (no difference), and the network's training kernels as early as nothing
+// else is to be won, weight gradients and reductions right after their wait, since
+// a step of few patches is a chain of ten short kernels (gradient of 1 patch 65 us,
+// 85 without; 32 110 / 120; 500 343 / 350).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 

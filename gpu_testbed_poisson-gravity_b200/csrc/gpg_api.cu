@@ -116,23 +116,28 @@ std::atomic<int> g_sor_variant[2][6] = {
 // set once a variant was chosen explicitly (gpg_set_sor_variant or the tuning
 // file): every launch then uses it, whatever its size
 std::atomic<bool> g_sor_pinned[2][6] = {};
-// Small launches: at a few thousand patches and fewer a launch leaves SMs
-// short of teams, and other layouts finish each patch sooner: those that split
-// each pair column between two lanes (twice the threads per patch), and for
-// FP64 ghost 4 the staged one.  Measured on B200 at 64-4096 patches per launch
-// (autotune.py --sizes, reference parameters, gravity), the variant below wins
-// up to max_npatch patches: FP32 ghost 1 at 256 patches 16.5 -> 12.4 us per
-// launch, ghost 2 16.0 -> 12.5, ghost 3 18.6 -> 16.6; FP32 ghost 5 runs the
-// large-launch layout at every size, ghost 4 the split column up to 1024 (45.6
-// us; the whole one 45.8, at 256 patches 20.6 and 22.7) and, with one patch per SM,
-// one row per lane (64 patches 14.5 -> 12.1, 100 16.5 -> 14.0; 200 18.6 -> 18.9).
-// FP64 ghost 2 at 256 53.6 -> 39.1, ghost 4 the staged kernel while each of its teams,
-// two per SM, has one patch (64 patches 67.1 -> 57.4, 148 68.6 -> 59.0, 296 85.8 ->
-// 81.5; 370 113 and 128).  FP64 ghost 5 keeps the
-// unstaged v11 up to 1024 patches: the staged kernel hands patches out at a
-// fixed stride, and 1024 patches over its 296 teams leave some teams a fourth
-// patch (333 vs 360 us; through the CUAPI path, 4 streams of 1024 patches,
-// 1.47 vs 1.55 ms of kernels per call).  Beyond it the table above holds.
+// Small launches: at a few thousand patches and fewer a launch leaves SMs short of
+// teams, and other layouts finish each patch sooner: those that split each pair
+// column between two lanes (twice the threads per patch), with one row per lane
+// instead of two twice as many again; at FP64 ghost 4 the staged kernel, whose teams
+// are as large but prefetch their inputs.  Each launch of up to max_npatch patches
+// runs the variant below.  Both sides, us per launch with gravity (autotune.py
+// --sizes, reference parameters; the variant below, then the one above the limit):
+//   FP32 1: 256 patches 10.2 / 14.1, 1480 19.8 / 21.4, 2048 27.6 / 28.0, 2368 30.8 / 30.3
+//        2: 256 10.2 / 13.2, 512 14.7 / 16.2, 740 17.0 / 18.7, 888 19.1 / 18.9
+//        3: 256 15.6 / 16.1, 444 19.3 / 20.0, 512 20.9 / 19.9
+//        4: v6, v11: 148 15.0 / 17.8, 200 20.1 / 20.0; v11, v13: 444 23.7 / 26.4, 740
+//           32.8 / 34.6, 888 44.4 / 36.3, 1024 46.7 / 45.8
+//        5: the large-launch layout at every size
+//   FP64 1: 256 30.3 / 33.1, 370 33.6 / 33.7; 2: 256 37.2 / 50.6, 444 45.1 / 52.5
+//        4: the staged kernel while each of its teams, two per SM, has one patch: 64
+//           57.4 / 67.1, 148 59.0 / 68.6, 296 81.6 / 86.1; 310 124.5 / 108.7
+//        5: 1024 337 / 348, 1184 384 / 353, but 888 292 / 266: the staged kernel hands
+//           patches out at a fixed stride, and 1024 patches over its 296 teams leave some
+//           teams a fourth patch, the size of the CUAPI path's four streams of 4096
+//           patches; below it the unstaged v11 costs 2 to 9 %
+// (512 at FP32 3 and 1024 at 4 were the crossings before the launches overlapped as
+// they do now; 148 and 296 are one and two patches per SM.)
 struct SorSmall {
   int max_npatch, variant;
 };

@@ -36,7 +36,7 @@
 // the cube and run the ordinary sweeps, stopping rule, output window and
 // (optionally) gravity update of sor_solve_patch_with.  Bound by the latency of a
 // batch's chain (interpolation, fold, MMAs, unfold, about one sweep) with 4 warps a
-// scheduler: 61 % of the issue slots; packing the transforms' instructions changed
+// scheduler: 60 % of the issue slots; packing the transforms' instructions changed
 // nothing.  The MMAs are issued by the whole of a half's first warp (one lane alone
 // takes 81 cycles an MMA for them, not 43; 306 -> 303 us).
 #pragma once

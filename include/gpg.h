@@ -263,8 +263,9 @@ GPG_API int gpg_batch_plan_destroy(gpg_batch_plan *plan);
  * tuning file ($GPG_TUNE_FILE, else sor_tune.txt beside libgpg.so, lines
  * "f32|f64 <ghost> <variant>") written by autotune.py.  Unless a variant was
  * chosen (by gpg_set_sor_variant or the tuning file), launches of up to a
- * stated number of patches (74 to 2048, per precision and ghost size) run a
- * small-batch variant instead, one that gives each patch more threads;
+ * stated number of patches (148 to 2048, per precision and ghost size) run a
+ * small-batch variant instead: one that gives each patch more threads, or for
+ * FP64 ghost 4 and 5 another form of the same layout (staged inputs, and none);
  * gpg_get_sor_variant reports the large-batch choice.
  * ------------------------------------------------------------------------- */
 GPG_API int gpg_sor_variant_count(void);
