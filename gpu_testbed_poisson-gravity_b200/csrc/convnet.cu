@@ -476,7 +476,8 @@ extern "C" int gpg_net_create(gpg_net **out, int max_batch, uint64_t seed, int d
     return nfail(GPG_ERR_CUDA, "upload: %s", cudaGetErrorString(e));
   }
   int rc = repack(n, 0);
-  if (!rc && cudaDeviceSynchronize() != cudaSuccess)
+  // the fills and the packing run on the default stream, which other streams need not follow
+  if (!rc && cudaStreamSynchronize(nullptr) != cudaSuccess)
     rc = nfail(GPG_ERR_CUDA, "set-up: %s", cudaGetErrorString(cudaGetLastError()));
   if (rc) {
     free_net(n);
@@ -514,7 +515,7 @@ extern "C" int gpg_net_set_params(gpg_net *n, const float *host) {
   NET_CUDA(cudaMemset(n->adam_v, 0, kParams * 4));
   n->step = 0;
   if (int rc = repack(n, 0)) return rc;
-  NET_CUDA(cudaDeviceSynchronize());
+  NET_CUDA(cudaStreamSynchronize(nullptr));
   return GPG_OK;
 }
 

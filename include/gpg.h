@@ -302,8 +302,9 @@ GPG_API int gpg_sor_variant_for_launch(int real_size, int ghost, int64_t npatch,
 typedef struct gpg_net gpg_net;
 /* every call on a net makes the net's device current, as the gpg_context
  * calls do; device arrays and streams passed to it belong to that device.
- * create, get_params and set_params wait for the device: calls on any stream
- * before them have ended, calls on any stream after them see the parameters */
+ * get_params and set_params wait for the device (so no stream may be capturing):
+ * calls on any stream before them have ended.  create and set_params return
+ * with the parameters in place for calls on any stream */
 GPG_API int gpg_net_create(gpg_net **net, int max_batch, uint64_t seed, int device_id);
 GPG_API int gpg_net_destroy(gpg_net *net);
 GPG_API int gpg_net_param_count(int64_t *count);
